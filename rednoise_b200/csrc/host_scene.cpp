@@ -5,6 +5,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <fstream>
+#include <limits>
 #include <map>
 #include <sstream>
 #include <thread>
@@ -479,8 +480,8 @@ void flatten_bvh4(const Bvh2 &bvh, DeviceLayout4 &out) {
 		int refs[4];
 		for (int k = 0; k < 4; k++) {
 			for (int a = 0; a < 3; a++) {
-				lo[a][k] = 1.0f;
-				hi[a][k] = -1.0f;
+				lo[a][k] = std::numeric_limits<float>::infinity();
+				hi[a][k] = -std::numeric_limits<float>::infinity();
 			}
 			refs[k] = 0;
 		}
@@ -502,10 +503,11 @@ void flatten_bvh4(const Bvh2 &bvh, DeviceLayout4 &out) {
 			}
 		}
 		F4 *o = &out.nodes[static_cast<size_t>(slot) * 8];
-		// (lo, hi) pairs per axis and entry, two entries per float4.
+		// Per axis a row of the four lo planes and a row of the four hi planes; an absent
+		// entry's box is empty (lo = +inf, hi = -inf), so no ray enters it.
 		for (int a = 0; a < 3; a++) {
-			o[2 * a] = {lo[a][0], hi[a][0], lo[a][1], hi[a][1]};
-			o[2 * a + 1] = {lo[a][2], hi[a][2], lo[a][3], hi[a][3]};
+			o[2 * a] = {lo[a][0], lo[a][1], lo[a][2], lo[a][3]};
+			o[2 * a + 1] = {hi[a][0], hi[a][1], hi[a][2], hi[a][3]};
 		}
 		o[6] = {as_float(refs[0]), as_float(refs[1]), as_float(refs[2]), as_float(refs[3])};
 		o[7] = {as_float(cnt), 0.0f, 0.0f, 0.0f};

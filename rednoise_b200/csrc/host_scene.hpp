@@ -114,8 +114,8 @@ void flatten_bvh(const TriangleSet &ts, const Bvh2 &bvh, DeviceLayout &out);
 // its parent's, so skipping the parent's test never admits a node the
 // reference would prune (rays with an infinite 1/d component excepted: those
 // use the 2-wide layout).
-// Node rows: [2a] = (lo_a[0], hi_a[0], lo_a[1], hi_a[1]), [2a+1] = entries 2, 3,
-// for axis a = x, y, z; [6] = refs[4]; [7] = (count, 0, 0, 0).
+// Node rows: [2a] = lo_a[4], [2a+1] = hi_a[4] for axis a = x, y, z (an absent entry's
+// box is empty: lo = +inf, hi = -inf); [6] = refs[4]; [7] = (count, 0, 0, 0).
 struct DeviceLayout4 {
 	std::vector<F4> nodes;
 	int root_ref = 0; // node index, or a leaf ref when the reference root is a leaf

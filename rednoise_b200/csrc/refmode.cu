@@ -348,7 +348,9 @@ __global__ void k_shade_scatter(DeferView dv) {
 	}
 }
 
-__global__ void __launch_bounds__(128) k_ref_shadow(SceneView sv, const RefParams *__restrict__ params, DeferView dv,
+// Eight blocks an SM: the 1.31M-triangle 1080p x 2 spp frame's shadow pass takes 12.2 ms,
+// against 12.7 at the 72 registers (seven blocks) it takes uncapped.
+__global__ void __launch_bounds__(128, 8) k_ref_shadow(SceneView sv, const RefParams *__restrict__ params, DeferView dv,
                                                     int *status) {
 	const RefParams &p = *params;
 	Ctx c{sv, nullptr, &p, 0};
