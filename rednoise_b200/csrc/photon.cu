@@ -6,16 +6,18 @@
 // path-dependent number more (a Fresnel choice at glass, a roulette draw and a
 // cosine direction at diffuse surfaces), so photon i starts where photon i-1's
 // draws ended. The GPU reproduces that sequence exactly, in parallel:
-//   1. the engine's first M outputs are generated on the host (M bounds the total);
+//   1. the engine's first M outputs are generated by one block;
 //   2. for EVERY position p < M a thread traces the photon that would start at p
 //      and records how many draws it takes, c(p), and how many photons it deposits;
 //   3. the chain s_0 = 0, s_{i+1} = s_i + c(s_i) is resolved by pointer doubling
 //      (jump tables next^(2^k)), giving each photon its start;
 //   4. deposit offsets are an exclusive scan over the chain, and the photons are
 //      traced again from their starts, writing deposits at the reference's indices.
+// M is first kFirstDrawsPerPhoton per photon, and kMaxDrawsPerPhoton (the bound no
+// photon exceeds) only where the chain turns out to run past that.
 // The uniform grid of cells of side `radius` becomes a stable sort of the deposits
-// by cell key, so a gather visits each cell's photons in insertion order and sums
-// them in the reference's order. Pass 2 shades every pixel (mirror, metal and
+// by cell key, with the deposits' records rewritten in that order, so a gather walks
+// each cell's photons in insertion order and sums them in the reference's order. Pass 2 shades every pixel (mirror, metal and
 // glass recursion on an explicit stack, direct light plus gathered irradiance at
 // diffuse hits); with final gather, each image row consumes its own
 // std::mt19937(1000 + y) stream in pixel order, one thread per row.
@@ -24,8 +26,6 @@
 #include <cub/cub.cuh>
 
 #include <algorithm>
-#include <random>
-#include <vector>
 
 #include "photon.hpp"
 #include "refshade.cuh"
@@ -36,6 +36,11 @@ namespace {
 
 constexpr int kPhotonDepth = 5;
 constexpr int kMaxDrawsPerPhoton = 2 + 3 * (kPhotonDepth + 1);
+// Positions tried first, per photon. A photon draws 2 numbers, then 1 at each diffuse
+// hit and 2 more when it goes on: 7 to 8 on average in rooms of albedo 0.5 to 0.8, 18
+// at the very most, so 10 covers all but mirror-white scenes at half the bound's work
+// (200 000 photons, 327 716 triangles: k_photon_counts 10.3 -> 5.0 ms).
+constexpr int kFirstDrawsPerPhoton = 10;
 constexpr int kMaxDepositsPerPhoton = kPhotonDepth + 1;
 constexpr float kEmitScale = 1.8f;
 
@@ -137,9 +142,68 @@ __device__ int trace_photon(const PhotonInput &in, uint32_t p0, float4 *out_pos,
 	return static_cast<int>(p - p0);
 }
 
-__global__ void __launch_bounds__(128) k_photon_counts(PhotonInput in, uint32_t n_pos, uint32_t *next,
+// The first n outputs of std::mt19937(seed), by one block of kMtThreads. The three
+// stretches of a generation (words 0..226, 227..453, 454..623) each read the previous
+// generation and words 227 earlier in this one; thread t takes words t, 227 + t and
+// 454 + t, so those are its own, and one barrier a generation suffices (word 623 also
+// reads this generation's word 0, which its thread forms again for itself). Bound by
+// that serial chain of n / 624 generations: 2.0 M outputs in 0.9 ms, where the host took
+// 8 ms for 4.0 M and the copy to the device 0.8 ms.
+constexpr int kMtThreads = 256;
+constexpr int kMtLag = 227; // 624 - 397
+__device__ __forceinline__ uint32_t mt_next(uint32_t a, uint32_t b, uint32_t far) {
+	const uint32_t y = (a & 0x80000000u) | (b & 0x7fffffffu);
+	return far ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
+}
+__device__ __forceinline__ uint32_t mt_temper(uint32_t y) {
+	y ^= y >> 11;
+	y ^= (y << 7) & 0x9d2c5680u;
+	y ^= (y << 15) & 0xefc60000u;
+	y ^= y >> 18;
+	return y;
+}
+__global__ void __launch_bounds__(kMtThreads) k_mt_stream(uint32_t seed, uint32_t n, uint32_t *__restrict__ out) {
+	__shared__ uint32_t gen[2][624];
+	const int t = threadIdx.x;
+	if (t == 0) {
+		uint32_t v = seed;
+		gen[0][0] = v;
+		for (int k = 1; k < 624; k++) {
+			v = 1812433253u * (v ^ (v >> 30)) + static_cast<uint32_t>(k);
+			gen[0][k] = v;
+		}
+	}
+	__syncthreads();
+	int cur = 0;
+	for (uint32_t base = 0; base < n; base += 624) {
+		const uint32_t *s = gen[cur];
+		uint32_t *d = gen[cur ^ 1];
+		if (t < kMtLag) {
+			const uint32_t w0 = mt_next(s[t], s[t + 1], s[t + 397]);
+			const uint32_t w1 = mt_next(s[t + kMtLag], s[t + kMtLag + 1], w0);
+			d[t] = w0;
+			d[t + kMtLag] = w1;
+			if (base + t < n)
+				out[base + t] = mt_temper(w0);
+			if (base + t + kMtLag < n)
+				out[base + t + kMtLag] = mt_temper(w1);
+			const int i = t + 2 * kMtLag;
+			if (i < 624) {
+				const uint32_t after = i < 623 ? s[i + 1] : mt_next(s[0], s[1], s[397]);
+				const uint32_t w2 = mt_next(s[i], after, w1);
+				d[i] = w2;
+				if (base + i < n)
+					out[base + i] = mt_temper(w2);
+			}
+		}
+		cur ^= 1;
+		__syncthreads();
+	}
+}
+
+__global__ void __launch_bounds__(128) k_photon_counts(PhotonInput in, uint32_t p0, uint32_t n_pos, uint32_t *next,
                                                        uint8_t *deposits, int *status) {
-	const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+	const uint32_t p = p0 + blockIdx.x * blockDim.x + threadIdx.x;
 	if (p >= n_pos)
 		return;
 	int err = 0, d = 0;
@@ -159,8 +223,9 @@ __global__ void k_jump_square(const uint32_t *__restrict__ jin, uint32_t *__rest
 	jout[p] = q < n_pos ? jin[q] : q;
 }
 
-// start[i] = next^i(0), from the binary digits of i.
-__global__ void k_chain_starts(const uint32_t *__restrict__ jumps, uint32_t n_pos, int levels, uint32_t n_photons,
+// start[i] = next^i(0), from the binary digits of i (a table per digit, stride entries apart).
+__global__ void k_chain_starts(const uint32_t *__restrict__ jumps, uint32_t n_pos, uint32_t stride, int levels,
+                               uint32_t n_photons,
                                const uint8_t *__restrict__ deposits, uint32_t *__restrict__ start,
                                uint32_t *__restrict__ count) {
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -169,7 +234,7 @@ __global__ void k_chain_starts(const uint32_t *__restrict__ jumps, uint32_t n_po
 	uint32_t pos = 0;
 	for (int k = 0; k < levels && pos < n_pos; k++)
 		if ((i >> k) & 1u)
-			pos = jumps[static_cast<size_t>(k) * n_pos + pos];
+			pos = jumps[static_cast<size_t>(k) * stride + pos];
 	start[i] = pos;
 	count[i] = pos < n_pos ? deposits[pos] : 0u;
 }
@@ -206,46 +271,72 @@ __global__ void k_photon_keys(const float4 *__restrict__ pos, uint32_t n, float 
 	idx[i] = i;
 }
 
+// The deposits' records in cell-key order.
+__global__ void k_photon_reorder(const uint32_t *__restrict__ idx, uint32_t n, const float4 *__restrict__ pos,
+                                 const float4 *__restrict__ pw, const float4 *__restrict__ dir,
+                                 float4 *__restrict__ spos, float4 *__restrict__ spw, float4 *__restrict__ sdir) {
+	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+	if (i >= n)
+		return;
+	const uint32_t j = idx[i];
+	spos[i] = pos[j];
+	spw[i] = pw[j];
+	sdir[i] = dir[j];
+}
+
 struct PhotonMapView {
 	const unsigned long long *keys; // sorted cell keys
-	const uint32_t *idx;            // photon index of each sorted entry (ascending within a cell)
-	const float4 *pos, *pw, *dir;
+	const float4 *pos, *pw, *dir;   // the deposits in that order (ascending insertion order within a cell)
 	uint32_t n;
 	float cell;
 	float radius;
 };
 
+__device__ __forceinline__ uint32_t first_key(const PhotonMapView &m, unsigned long long key) {
+	uint32_t lo = 0, hi = m.n;
+	while (lo < hi) {
+		const uint32_t mid = (lo + hi) >> 1;
+		if (__ldg(m.keys + mid) < key)
+			lo = mid + 1;
+		else
+			hi = mid;
+	}
+	return lo;
+}
+
 // PhotonMap::gather (src/Photon.cpp:21-46): the 27 cells in the reference's loop
-// order, each cell's photons in insertion order.
+// order, each cell's photons in insertion order. The z coordinate is the key's lowest
+// field, so the three cells of one (x, y) are one stretch of the sorted records (unless
+// z + 1 or z - 1 wraps around the field: then they are looked up one by one).
+// A pixel tests some ten thousand photons, whose records its warp's neighbours share: the
+// loop is bound by issue. Walking indices into unsorted records, with a key compare per
+// photon and the accepted photons' loads behind a branch, serialised four dependent
+// loads per photon; on sorted records every load's address is known ahead and nothing
+// branches (200 000 photons, 1280 x 720: 181 -> 51 ms).
 __device__ V3 gather(const PhotonMapView &m, V3 point, V3 normal) {
 	const int cx = cell_coord(point.x, m.cell), cy = cell_coord(point.y, m.cell), cz = cell_coord(point.z, m.cell);
 	V3 sum = mk(0.0f, 0.0f, 0.0f);
 	const float r2 = m.radius * m.radius;
-	for (int dx = -1; dx <= 1; dx++)
-		for (int dy = -1; dy <= 1; dy++)
-			for (int dz = -1; dz <= 1; dz++) {
-				const unsigned long long key = static_cast<unsigned long long>(cell_key(cx + dx, cy + dy, cz + dz));
-				uint32_t lo = 0, hi = m.n;
-				while (lo < hi) {
-					const uint32_t mid = (lo + hi) >> 1;
-					if (m.keys[mid] < key)
-						lo = mid + 1;
-					else
-						hi = mid;
-				}
-				for (uint32_t e = lo; e < m.n && m.keys[e] == key; e++) {
-					const uint32_t pi = m.idx[e];
-					const float4 pp = m.pos[pi];
-					const V3 d = mk(pp.x, pp.y, pp.z) - point;
-					if (dot(d, d) > r2)
-						continue;
-					const float4 pd = m.dir[pi];
-					if (dot(normal, -mk(pd.x, pd.y, pd.z)) <= 0.0f)
-						continue;
-					const float4 pw = m.pw[pi];
-					sum = sum + mk(pw.x, pw.y, pw.z);
-				}
+	const int zf = (cz + (1 << 20)) & 0x1FFFFF;
+	const bool wraps = zf == 0 || zf == 0x1FFFFF;
+	const int runs = wraps ? 27 : 9;
+	for (int run = 0; run < runs; run++) {
+		const int column = wraps ? run / 3 : run;
+		const int x = cx + column / 3 - 1, y = cy + column % 3 - 1;
+		const int z0 = wraps ? cz + run % 3 - 1 : cz - 1, z1 = wraps ? z0 : cz + 1;
+		const uint32_t lo = first_key(m, static_cast<unsigned long long>(cell_key(x, y, z0)));
+		const uint32_t hi = first_key(m, static_cast<unsigned long long>(cell_key(x, y, z1)) + 1);
+#pragma unroll 4
+		for (uint32_t e = lo; e < hi; e++) {
+			const float4 pp = __ldg(m.pos + e), pd = __ldg(m.dir + e), pw = __ldg(m.pw + e);
+			const V3 d = mk(pp.x, pp.y, pp.z) - point;
+			if (!(dot(d, d) > r2) && !(dot(normal, -mk(pd.x, pd.y, pd.z)) <= 0.0f)) {
+				sum.x = sum.x + pw.x;
+				sum.y = sum.y + pw.y;
+				sum.z = sum.z + pw.z;
 			}
+		}
+	}
 	return sum / (3.14159265f * r2);
 }
 
@@ -397,14 +488,17 @@ __device__ V3 photon_camera_dir(const RefParams &p, int x, int y) {
 __global__ void __launch_bounds__(128) k_photon_pixels(SceneView sv, const float4 *__restrict__ ref_shade,
                                                        const RefParams *__restrict__ params, PhotonMapView m,
                                                        uint32_t *__restrict__ argb, int *status) {
+	// a warp takes an 8 x 4 pixel tile, a block 16 x 8: its gathers meet the same cells
 	const RefParams &p = *params;
-	const long pix = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
-	if (pix >= static_cast<long>(p.width) * p.height)
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const int tiles_x = (p.width + 15) / 16;
+	const int x = static_cast<int>(blockIdx.x) % tiles_x * 16 + (warp & 1) * 8 + (lane & 7);
+	const int y = static_cast<int>(blockIdx.x) / tiles_x * 8 + (warp >> 1) * 4 + (lane >> 3);
+	if (x >= p.width || y >= p.height)
 		return;
-	const int x = static_cast<int>(pix % p.width), y = static_cast<int>(pix / p.width);
 	Ctx c{sv, ref_shade, &p, 0};
 	const V3 colour = photon_shade(c, m, l3(p.position), photon_camera_dir(p, x, y), 0, nullptr) * 255.0f;
-	argb[pix] = pack_pixel(colour);
+	argb[static_cast<size_t>(y) * p.width + x] = pack_pixel(colour);
 	if (c.err)
 		atomicOr(status, 1);
 }
@@ -430,6 +524,11 @@ __global__ void __launch_bounds__(64) k_photon_rows(SceneView sv, const float4 *
 
 inline size_t align256(size_t b) { return (b + 255) & ~static_cast<size_t>(255); }
 
+// The jump tables' memory; once the starts are known it holds the sorted deposit records.
+inline size_t jump_bytes(size_t max_pos, int levels, size_t n_dep) {
+	return std::max(align256(max_pos * 4) * static_cast<size_t>(levels), 3 * align256(n_dep * 16));
+}
+
 } // namespace
 
 cudaError_t photon_scratch_bytes(int n_photons, size_t &bytes) {
@@ -450,7 +549,7 @@ cudaError_t photon_scratch_bytes(int n_photons, size_t &bytes) {
 	                                  static_cast<uint32_t *>(nullptr), n_photons + 1);
 	if (e != cudaSuccess)
 		return e;
-	bytes = align256(n_draws * 4) + align256(n_pos * 4) * static_cast<size_t>(levels) + align256(n_pos) +
+	bytes = align256(n_draws * 4) + jump_bytes(n_pos, levels, n_dep) + align256(n_pos) +
 	        3 * align256((static_cast<size_t>(n_photons) + 1) * 4) + 3 * align256(n_dep * 16) +
 	        2 * align256(n_dep * 8) + 2 * align256(n_dep * 4) + align256(std::max(cub_bytes, scan_bytes)) + 1024;
 	return cudaSuccess;
@@ -460,8 +559,7 @@ cudaError_t launch_photon_mapped(const SceneView &sv, const float4 *ref_shade, c
                                  const RefParams *d_params, int n_photons, int gather_rays, void *scratch,
                                  size_t scratch_bytes, uint32_t *argb, int *status, cudaStream_t st,
                                  unsigned *deposits_out) {
-	const size_t n_pos = static_cast<size_t>(n_photons) * kMaxDrawsPerPhoton + 8;
-	const size_t n_draws = n_pos + kMaxDrawsPerPhoton + 8;
+	const size_t max_pos = static_cast<size_t>(n_photons) * kMaxDrawsPerPhoton + 8;
 	int levels = 1;
 	while ((1ull << levels) < static_cast<unsigned long long>(n_photons))
 		levels++;
@@ -473,9 +571,13 @@ cudaError_t launch_photon_mapped(const SceneView &sv, const float4 *ref_shade, c
 		b += align256(bytes);
 		return p;
 	};
-	uint32_t *d_draws = reinterpret_cast<uint32_t *>(take(n_draws * 4));
-	uint32_t *d_jumps = reinterpret_cast<uint32_t *>(take(n_pos * 4 * static_cast<size_t>(levels)));
-	uint8_t *d_dep = reinterpret_cast<uint8_t *>(take(n_pos));
+	uint32_t *d_draws = reinterpret_cast<uint32_t *>(take((max_pos + kMaxDrawsPerPhoton + 8) * 4));
+	char *jump_mem = take(jump_bytes(max_pos, levels, n_dep));
+	uint32_t *d_jumps = reinterpret_cast<uint32_t *>(jump_mem);
+	float4 *s_pos = reinterpret_cast<float4 *>(jump_mem);
+	float4 *s_pw = reinterpret_cast<float4 *>(jump_mem + align256(n_dep * 16));
+	float4 *s_dir = reinterpret_cast<float4 *>(jump_mem + 2 * align256(n_dep * 16));
+	uint8_t *d_dep = reinterpret_cast<uint8_t *>(take(max_pos));
 	uint32_t *d_start = reinterpret_cast<uint32_t *>(take((static_cast<size_t>(n_photons) + 1) * 4));
 	uint32_t *d_count = reinterpret_cast<uint32_t *>(take((static_cast<size_t>(n_photons) + 1) * 4));
 	uint32_t *d_off = reinterpret_cast<uint32_t *>(take((static_cast<size_t>(n_photons) + 1) * 4));
@@ -492,14 +594,6 @@ cudaError_t launch_photon_mapped(const SceneView &sv, const float4 *ref_shade, c
 		return cudaErrorInvalidValue;
 	const size_t tmp_bytes = scratch_bytes - used;
 
-	// 1. the engine's outputs: std::mt19937(777), as the reference seeds it
-	std::vector<uint32_t> draws(n_draws);
-	std::mt19937 gen(777u);
-	for (size_t i = 0; i < n_draws; i++)
-		draws[i] = static_cast<uint32_t>(gen());
-	cudaError_t e = cudaMemcpyAsync(d_draws, draws.data(), n_draws * 4, cudaMemcpyHostToDevice, st);
-	if (e != cudaSuccess)
-		return e;
 	// the emitting light: the first light (src/Renderer.cpp:1315-1323)
 	const RefLight &L = hp.lights[0];
 	PhotonInput in;
@@ -510,32 +604,46 @@ cudaError_t launch_photon_mapped(const SceneView &sv, const float4 *ref_shade, c
 	const float scale = L.intensity * kEmitScale / static_cast<float>(n_photons);
 	in.power = V3{L.colour[0] * scale, L.colour[1] * scale, L.colour[2] * scale};
 
-	// 2. draws and deposits of a photon starting at every position
 	const int bs = 128;
-	k_photon_counts<<<ceil_div(static_cast<long>(n_pos), bs), bs, 0, st>>>(in, static_cast<uint32_t>(n_pos), d_jumps,
-	                                                                        d_dep, status);
-	// 3. jump tables next^(2^k), then every photon's start
-	for (int k = 1; k < levels; k++)
-		k_jump_square<<<ceil_div(static_cast<long>(n_pos), 256), 256, 0, st>>>(
-		    d_jumps + static_cast<size_t>(k - 1) * n_pos, d_jumps + static_cast<size_t>(k) * n_pos,
-		    static_cast<uint32_t>(n_pos));
-	k_chain_starts<<<ceil_div(static_cast<long>(n_photons), 256), 256, 0, st>>>(
-	    d_jumps, static_cast<uint32_t>(n_pos), levels, static_cast<uint32_t>(n_photons), d_dep, d_start, d_count);
-	e = cudaMemsetAsync(d_count + n_photons, 0, 4, st);
-	if (e != cudaSuccess)
-		return e;
-	// 4. deposit offsets, then the photons themselves
-	size_t tb = tmp_bytes;
-	e = cub::DeviceScan::ExclusiveSum(d_tmp, tb, d_count, d_off, n_photons + 1, st);
-	if (e != cudaSuccess)
-		return e;
 	uint32_t n_total = 0;
-	e = cudaMemcpyAsync(&n_total, d_off + n_photons, 4, cudaMemcpyDeviceToHost, st);
-	if (e != cudaSuccess)
-		return e;
-	e = cudaStreamSynchronize(st);
-	if (e != cudaSuccess)
-		return e;
+	cudaError_t e = cudaSuccess;
+	size_t tried = 0; // positions whose draw counts are known
+	for (const size_t n_pos : {std::min(max_pos, static_cast<size_t>(n_photons) * kFirstDrawsPerPhoton + 64), max_pos}) {
+		// 1. the engine's outputs: std::mt19937(777), as the reference seeds it
+		k_mt_stream<<<1, kMtThreads, 0, st>>>(777u, static_cast<uint32_t>(n_pos + kMaxDrawsPerPhoton + 8), d_draws);
+		// 2. draws and deposits of a photon starting at every position
+		k_photon_counts<<<ceil_div(static_cast<long>(n_pos - tried), bs), bs, 0, st>>>(
+		    in, static_cast<uint32_t>(tried), static_cast<uint32_t>(n_pos), d_jumps, d_dep, status);
+		tried = n_pos;
+		// 3. jump tables next^(2^k), then every photon's start
+		for (int k = 1; k < levels; k++)
+			k_jump_square<<<ceil_div(static_cast<long>(n_pos), 256), 256, 0, st>>>(
+			    d_jumps + static_cast<size_t>(k - 1) * max_pos, d_jumps + static_cast<size_t>(k) * max_pos,
+			    static_cast<uint32_t>(n_pos));
+		k_chain_starts<<<ceil_div(static_cast<long>(n_photons), 256), 256, 0, st>>>(
+		    d_jumps, static_cast<uint32_t>(n_pos), static_cast<uint32_t>(max_pos), levels,
+		    static_cast<uint32_t>(n_photons), d_dep, d_start, d_count);
+		e = cudaMemsetAsync(d_count + n_photons, 0, 4, st);
+		if (e != cudaSuccess)
+			return e;
+		// 4. deposit offsets, then the photons themselves
+		size_t tb = tmp_bytes;
+		e = cub::DeviceScan::ExclusiveSum(d_tmp, tb, d_count, d_off, n_photons + 1, st);
+		if (e != cudaSuccess)
+			return e;
+		uint32_t last = 0; // the last photon's start: past the table when the chain ran out of it
+		e = cudaMemcpyAsync(&n_total, d_off + n_photons, 4, cudaMemcpyDeviceToHost, st);
+		if (e != cudaSuccess)
+			return e;
+		e = cudaMemcpyAsync(&last, d_start + n_photons - 1, 4, cudaMemcpyDeviceToHost, st);
+		if (e != cudaSuccess)
+			return e;
+		e = cudaStreamSynchronize(st);
+		if (e != cudaSuccess)
+			return e;
+		if (last < n_pos)
+			break;
+	}
 	if (deposits_out)
 		*deposits_out = n_total;
 	k_photon_deposit<<<ceil_div(static_cast<long>(n_photons), bs), bs, 0, st>>>(in, static_cast<uint32_t>(n_photons),
@@ -544,31 +652,29 @@ cudaError_t launch_photon_mapped(const SceneView &sv, const float4 *ref_shade, c
 	// the grid: a stable sort of the deposits by cell key
 	const float radius = 0.25f;
 	PhotonMapView m{};
-	m.pos = d_pos;
-	m.pw = d_pw;
-	m.dir = d_dir;
+	m.keys = d_k1;
+	m.pos = s_pos;
+	m.pw = s_pw;
+	m.dir = s_dir;
 	m.n = n_total;
 	m.cell = radius;
 	m.radius = radius;
 	if (n_total > 0) {
 		k_photon_keys<<<ceil_div(static_cast<long>(n_total), 256), 256, 0, st>>>(d_pos, n_total, radius, d_k0, d_i0);
-		tb = tmp_bytes;
+		size_t tb = tmp_bytes;
 		e = cub::DeviceRadixSort::SortPairs(d_tmp, tb, d_k0, d_k1, d_i0, d_i1, static_cast<int>(n_total), 0, 64, st);
 		if (e != cudaSuccess)
 			return e;
-		m.keys = d_k1;
-		m.idx = d_i1;
-	} else {
-		m.keys = d_k0;
-		m.idx = d_i0;
+		k_photon_reorder<<<ceil_div(static_cast<long>(n_total), 256), 256, 0, st>>>(d_i1, n_total, d_pos, d_pw, d_dir,
+		                                                                            s_pos, s_pw, s_dir);
 	}
 	// pass 2
-	const long npix = static_cast<long>(hp.width) * hp.height;
 	if (gather_rays > 0)
 		k_photon_rows<<<ceil_div(static_cast<long>(hp.height), 64), 64, 0, st>>>(sv, ref_shade, d_params, m,
 		                                                                         gather_rays, argb, status);
 	else
-		k_photon_pixels<<<ceil_div(npix, bs), bs, 0, st>>>(sv, ref_shade, d_params, m, argb, status);
+		k_photon_pixels<<<static_cast<unsigned>((hp.width + 15) / 16) * static_cast<unsigned>((hp.height + 7) / 8), 128,
+		                  0, st>>>(sv, ref_shade, d_params, m, argb, status);
 	return cudaGetLastError();
 }
 
