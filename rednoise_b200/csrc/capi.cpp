@@ -345,7 +345,7 @@ rn_status rn_pt_render_photon_mapped(rn_scene *scene, const rn_pt_ref_params *pr
 			p.lights[i] = to_ref_light(prm->lights[i]);
 	}
 	size_t map_bytes = 0;
-	RNB_CUDA(photon_scratch_bytes(num_photons, map_bytes));
+	RNB_CUDA(photon_scratch_bytes(num_photons, prm->width, prm->height, map_bytes));
 	cudaStream_t cs = pick_stream(scene, stream);
 	std::lock_guard<std::mutex> lock(scene->scratch_mu);
 	const size_t pb = (sizeof(RefParams) + 255) & ~size_t(255);

@@ -10,8 +10,8 @@ namespace rnb {
 
 constexpr int kMaxPhotons = 1 << 22;
 
-// Device scratch the photon mapper needs for n_photons photons.
-cudaError_t photon_scratch_bytes(int n_photons, size_t &bytes);
+// Device scratch the photon mapper needs for n_photons photons and an image of that size.
+cudaError_t photon_scratch_bytes(int n_photons, int width, int height, size_t &bytes);
 
 // Both passes of renderPhotonMapped into argb (device, width*height 0xAARRGGBB).
 // hp: host copy of the parameters (lights[0] emits); d_params: the same on the
