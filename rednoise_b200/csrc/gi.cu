@@ -118,7 +118,7 @@ __device__ __forceinline__ V3 tri_albedo(const float4 *ref_shade, int idx) {
 __device__ __forceinline__ Hit intersect_alone(Ctx &c, V3 o, V3 d) {
 	const RayPre r = make_ray(o.x, o.y, o.z, d.x, d.y, d.z);
 	HitRec h;
-	if (c.sv.nodes4 && finite_inverse(r)) {
+	if (c.sv.nodes4 && bounded_ray(c.sv, r)) {
 		LocalStack<unsigned long long> st;
 		h = trace_closest4_flat(c.sv, r, -1, c.err, st);
 	} else {

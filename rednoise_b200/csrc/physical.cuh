@@ -74,7 +74,7 @@ __device__ __forceinline__ F3 cross3(F3 a, F3 b) {
 }
 // 1 / sqrt with IEEE division and square root (not the approximate rsqrtf), so a
 // unit vector carries the same bits as the CPU restatement's a * (1 / std::sqrt(a.a)).
-__device__ __forceinline__ F3 norm3(F3 a) { return a * (1.0f / sqrtf(dot3(a, a))); }
+__device__ __forceinline__ F3 norm3(F3 a) { return a * inv_sqrt_exact(dot3(a, a)); }
 __device__ __forceinline__ float maxc(F3 a) { return fmaxf(a.x, fmaxf(a.y, a.z)); }
 __device__ __forceinline__ F3 ld3(const float4 v) { return {v.x, v.y, v.z}; }
 

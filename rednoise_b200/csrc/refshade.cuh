@@ -37,9 +37,9 @@ __device__ __forceinline__ float dot(V3 a, V3 b) {
 __device__ __forceinline__ V3 cross(V3 x, V3 y) {
 	return {x.y * y.z - y.y * x.z, x.z * y.x - y.z * x.x, x.x * y.y - y.x * x.y};
 }
-__device__ __forceinline__ float length(V3 v) { return sqrtf(dot(v, v)); }
+__device__ __forceinline__ float length(V3 v) { return sqrt_exact(dot(v, v)); }
 // glm normalize: v * inversesqrt(dot(v, v)), inversesqrt = 1 / sqrt(x)
-__device__ __forceinline__ V3 normalize(V3 v) { return v * (1.0f / sqrtf(dot(v, v))); }
+__device__ __forceinline__ V3 normalize(V3 v) { return v * inv_sqrt_exact(dot(v, v)); }
 // glm reflect: I - N * dot(N, I) * 2
 __device__ __forceinline__ V3 reflect(V3 I, V3 N) { return I - (N * dot(N, I)) * 2.0f; }
 // glm refract

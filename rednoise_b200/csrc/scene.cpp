@@ -1,4 +1,5 @@
 // rn_scene lifetime, lazy device preparation and the ray-query entry points.
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <cmath>
@@ -153,6 +154,14 @@ rn_status prepare_scene(rn_scene *s) {
 	v.n_tris = n;
 	v.n_nodes = lay.internal_count;
 	v.n_nodes4 = static_cast<int>(lay4.nodes.size() / 8);
+	// directions up to max_dir keep 6 max|d| max|e|^2 (the triangle test's determinant) below 2^126
+	double edge = 0.0;
+	for (size_t i = 0; i < static_cast<size_t>(n); i++)
+		for (int a = 0; a < 3; a++) {
+			const float *t = &ts.v[9 * i + static_cast<size_t>(a)];
+			edge = std::max({edge, std::fabs(static_cast<double>(t[3]) - t[0]), std::fabs(static_cast<double>(t[6]) - t[0])});
+		}
+	v.max_dir = edge > 0.0 ? static_cast<float>(std::min(3.0e38, std::ldexp(1.0, 123) / (edge * edge))) : 3.0e38f;
 	s->view = v;
 	s->prepared = true;
 	return RN_OK;

@@ -24,6 +24,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "rounded.cuh"
 
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -43,6 +44,9 @@ struct SceneView {
 	int n_tris;
 	int n_nodes;  // internal nodes of the 2-wide layout
 	int n_nodes4; // nodes of the 4-wide layout (0 when absent)
+	// |det| <= 6 max|d| max|e|^2 in the triangle test: directions with components below
+	// max_dir keep it under 2^126
+	float max_dir;
 };
 
 struct RayPre {
@@ -69,9 +73,15 @@ __device__ __forceinline__ RayPre make_ray(float ox, float oy, float oz, float d
 	r.dx = dx;
 	r.dy = dy;
 	r.dz = dz;
-	r.ix = __fdiv_rn(1.0f, dx);
-	r.iy = __fdiv_rn(1.0f, dy);
-	r.iz = __fdiv_rn(1.0f, dz);
+	r.ix = rcp_bounded(dx);
+	r.iy = rcp_bounded(dy);
+	r.iz = rcp_bounded(dz);
+	const float ax = fabsf(dx), ay = fabsf(dy), az = fabsf(dz);
+	if (!(fminf(ax, fminf(ay, az)) >= 0x1p-126f && fmaxf(ax, fmaxf(ay, az)) < 0x1p126f)) { // a zero, say
+		r.ix = __fdiv_rn(1.0f, dx);
+		r.iy = __fdiv_rn(1.0f, dy);
+		r.iz = __fdiv_rn(1.0f, dz);
+	}
 	r.ndx = -dx;
 	r.ndy = -dy;
 	r.ndz = -dz;
@@ -113,7 +123,10 @@ __device__ __forceinline__ bool slab(float lox, float hix, float loy, float hiy,
 
 // Reference ray/triangle test on a stored (v0, e0 = v1 - v0, e1 = v2 - v0)
 // record; e0/e1 were computed on the host with the same IEEE subtraction the
-// reference performs at test time, so they carry the same bits.
+// reference performs at test time, so they carry the same bits. kBounded: the ray is a
+// bounded_ray of the scene, whose determinants stay in rcp_bounded's range (those below
+// 1e-8 are rejected whatever their reciprocal).
+template <bool kBounded = false>
 __device__ __forceinline__ bool tri_test(const float4 a, const float4 b, const float4 c, const RayPre &r, float &t,
                                          float &u, float &v) {
 	const float spx = __fsub_rn(r.ox, a.x);
@@ -126,7 +139,7 @@ __device__ __forceinline__ bool tri_test(const float4 a, const float4 b, const f
 	const float det = __fadd_rn(__fsub_rn(__fmul_rn(r.ndx, c00), __fmul_rn(b.x, A)), __fmul_rn(c.x, B));
 	if (fabsf(det) < 1e-8f)
 		return false;
-	const float k = __fdiv_rn(1.0f, det);
+	const float k = kBounded ? rcp_bounded(det) : __fdiv_rn(1.0f, det);
 	// Row 1 of the inverse gives u.
 	const float i01 = __fmul_rn(-A, k);
 	const float i11 = __fmul_rn(__fsub_rn(__fmul_rn(r.ndx, c.z), __fmul_rn(c.x, r.ndz)), k);
@@ -470,8 +483,13 @@ __device__ __forceinline__ unsigned long long pack_entry(int ref, float tenter) 
 }
 
 __device__ __forceinline__ bool finite_inverse(const RayPre &r) {
-	return fabsf(r.ix) < __int_as_float(0x7f800000) && fabsf(r.iy) < __int_as_float(0x7f800000) &&
-	       fabsf(r.iz) < __int_as_float(0x7f800000);
+	const float inf = __int_as_float(0x7f800000);
+	return (fabsf(r.ix) < inf) & (fabsf(r.iy) < inf) & (fabsf(r.iz) < inf);
+}
+// Rays for the 4-wide tree: a finite inverse direction, and a direction
+// short enough that no determinant leaves rcp_bounded's range (SceneView::max_dir).
+__device__ __forceinline__ bool bounded_ray(const SceneView &s, const RayPre &r) {
+	return finite_inverse(r) & (fmaxf(fabsf(r.dx), fmaxf(fabsf(r.dy), fabsf(r.dz))) < s.max_dir);
 }
 
 // Traversal stack storage. LocalStack keeps the whole stack in the thread's
@@ -744,7 +762,7 @@ __device__ __forceinline__ HitRec trace_closest4_spec(const SceneView &s, const 
 					const float4 b = __ldg(tp + 1);
 					const float4 c = __ldg(tp + 2);
 					float t, u, v;
-					if (tri_test(a, b, c, r, t, u, v) && t < h.t) {
+					if (tri_test<true>(a, b, c, r, t, u, v) && t < h.t) {
 						h.idx = ti;
 						h.t = t;
 						h.u = u;
@@ -833,7 +851,7 @@ __device__ __forceinline__ bool trace_any4_spec(const SceneView &s, const RayPre
 				const float4 b = __ldg(tp + 1);
 				const float4 c = __ldg(tp + 2);
 				float t, u, v;
-				if (tri_test(a, b, c, r, t, u, v) && t < tmax)
+				if (tri_test<true>(a, b, c, r, t, u, v) && t < tmax)
 					return true;
 			}
 			leaf = kNoRef;
@@ -946,7 +964,7 @@ __device__ __forceinline__ bool trav_step(TravState &ts, const SceneView &s, int
 		const float4 bb = __ldg(tp + 1);
 		const float4 c = __ldg(tp + 2);
 		float t, u, v;
-		if (!tri_test(a, bb, c, ts.r, t, u, v))
+		if (!tri_test<true>(a, bb, c, ts.r, t, u, v))
 			continue;
 		if (kAny) {
 			if (t < ts.tmax) {
@@ -971,7 +989,7 @@ __device__ __forceinline__ bool trav_step(TravState &ts, const SceneView &s, int
 // and the any-hit stage from 40.3 to 36.6 ms, images unchanged.
 template <int kOrder>
 __device__ __forceinline__ HitRec trace_closest_best(const SceneView &s, const RayPre &r, int ignore, int &err) {
-	if (kOrder == kOrderReference && s.nodes4 && finite_inverse(r)) {
+	if (kOrder == kOrderReference && s.nodes4 && bounded_ray(s, r)) {
 		LocalStack<unsigned long long> st;
 		return trace_closest4_spec(s, r, ignore, err, st);
 	}
@@ -979,7 +997,7 @@ __device__ __forceinline__ HitRec trace_closest_best(const SceneView &s, const R
 }
 
 __device__ __forceinline__ bool trace_any_best(const SceneView &s, const RayPre &r, float tmax, int ignore, int &err) {
-	if (s.nodes4 && finite_inverse(r)) {
+	if (s.nodes4 && bounded_ray(s, r)) {
 		LocalStack<int> st;
 		return trace_any4_spec(s, r, tmax, ignore, err, st);
 	}
@@ -990,14 +1008,14 @@ __device__ __forceinline__ bool trace_any_best(const SceneView &s, const RayPre 
 template <int kOrder, class Stack>
 __device__ __forceinline__ HitRec trace_closest_best(const SceneView &s, const RayPre &r, int ignore, int &err,
                                                      Stack &st) {
-	if (kOrder == kOrderReference && s.nodes4 && finite_inverse(r))
+	if (kOrder == kOrderReference && s.nodes4 && bounded_ray(s, r))
 		return trace_closest4_spec(s, r, ignore, err, st);
 	return trace_closest<kOrder>(s, r, ignore, err);
 }
 template <class Stack>
 __device__ __forceinline__ bool trace_any_best(const SceneView &s, const RayPre &r, float tmax, int ignore, int &err,
                                                Stack &st) {
-	if (s.nodes4 && finite_inverse(r))
+	if (s.nodes4 && bounded_ray(s, r))
 		return trace_any4_spec(s, r, tmax, ignore, err, st);
 	return trace_any(s, r, tmax, ignore, err);
 }

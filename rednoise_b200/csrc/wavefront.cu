@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(128) k_wf_trace_dyn(const WfJob *__restrict__ 
 						ignore = __float_as_int(o.w);
 					}
 					jb = jobs + (only_job >= 0 ? only_job : __float_as_int(pool.L[slot].w));
-					if (jb->sc.sv.nodes4 && finite_inverse(r)) {
+					if (jb->sc.sv.nodes4 && bounded_ray(jb->sc.sv, r)) {
 						trav_begin<kAny>(ts, jb->sc.sv, r, tmax, ignore);
 						active = true;
 					} else if (kAny) { // rays with an infinite 1/d component: 2-wide path at once
