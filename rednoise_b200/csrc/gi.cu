@@ -6,12 +6,13 @@
 // Bidirectional, reference stream: every image row draws from its own
 // std::mt19937(9871 + y) in the reference's order, so the canvas equals the
 // reference's. The number of draws a sample takes depends on its subpath lengths,
-// so a row's samples are found in stream order: one thread per row traces the
-// camera and light subpaths (the closest-hit chain) and records their vertices;
-// then the connections (the shadow rays, most of the work) run one thread per
-// connection and are summed per pixel in the reference's order. Columns are processed in chunks so
-// the vertex records stay within a fixed budget; the row streams persist in
-// device memory between chunks.
+// so where a sample's draws start depends on every sample before it in its row. A
+// block per row traces the camera and light subpaths of the samples that would start
+// at each of the next stream positions, side by side, then follows the chain of the
+// positions that are really taken and records those samples' vertices; then the
+// connections (the shadow rays) run one thread per connection and are summed per pixel
+// in the reference's order. Columns are processed in chunks so the vertex records stay
+// within a fixed budget; the row streams persist in device memory between chunks.
 //
 // Bidirectional, counter stream: the same estimator with each (pixel, sample)
 // drawing from Philox-4x32-10 under the seed; the subpaths are traced one thread
@@ -44,34 +45,8 @@ constexpr float kGiEps = 1e-3f;
 constexpr float kGiLightHalf = 0.18f;
 constexpr int kGiMaxDepth = 4;
 constexpr int kMltDims = 2 + 4 * kGiMaxDepth;
-constexpr int kRowsPerBlock = 1;
 
 __device__ __forceinline__ float gi_light_area() { return (2.0f * kGiLightHalf) * (2.0f * kGiLightHalf); }
-
-// std::mt19937 of one image row kept in device memory: 624 contiguous words, so
-// the row's lone thread finds its state in a few cache lines.
-struct MtRow {
-	uint32_t *s;
-	int i;
-	__device__ void twist() {
-		for (int k = 0; k < 624; k++) {
-			const uint32_t y = (s[k] & 0x80000000u) | (s[k + 1 < 624 ? k + 1 : 0] & 0x7fffffffu);
-			const int m = k + 397 < 624 ? k + 397 : k + 397 - 624;
-			s[k] = s[m] ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
-		}
-		i = 0;
-	}
-	__device__ float operator()() {
-		if (i >= 624)
-			twist();
-		uint32_t y = s[i++];
-		y ^= y >> 11;
-		y ^= (y << 7) & 0x9d2c5680u;
-		y ^= (y << 15) & 0xefc60000u;
-		y ^= y >> 18;
-		return canonical01(y);
-	}
-};
 
 __device__ __forceinline__ uint32_t u4_word(U4 v, int k) { return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w; }
 
@@ -88,6 +63,7 @@ struct CtrDraw {
 		n++;
 		return canonical01(u4_word(blk, w));
 	}
+	__device__ V3 local();
 };
 
 struct GV {
@@ -113,75 +89,87 @@ __device__ __forceinline__ V3 tri_albedo(const float4 *ref_shade, int idx) {
 	return mk(s1.x, s1.y, s1.z) / 255.0f;
 }
 
-// Closest hit for a thread that runs alone (the row pass): the same result as
-// intersect(), with each leaf's triangle tests overlapped.
-__device__ __forceinline__ Hit intersect_alone(Ctx &c, V3 o, V3 d) {
-	const RayPre r = make_ray(o.x, o.y, o.z, d.x, d.y, d.z);
-	HitRec h;
-	if (c.sv.nodes4 && bounded_ray(c.sv, r)) {
-		LocalStack<unsigned long long> st;
-		h = trace_closest4_flat(c.sv, r, -1, c.err, st);
-	} else {
-		h = trace_closest<kOrderReference>(c.sv, r, -1, c.err);
-	}
-	Hit out;
-	out.hit = h.idx >= 0;
-	out.idx = h.idx;
-	out.t = h.t;
-	out.point = o + h.t * d;
-	return out;
+// cosineHemisphere (src/Renderer.cpp:85-96) in two halves: the direction's coordinates, which
+// depend on the two random numbers alone, and the frame, which depends on the normal.
+__device__ __forceinline__ V3 hemisphere_local(float u1, float u2) {
+	const float r = sqrtf(u1);
+	const float theta = 2.0f * 3.14159265f * u2;
+	return mk(r * lm_cos(theta), r * lm_sin(theta), sqrtf(smax(0.0f, 1.0f - u1)));
+}
+__device__ __forceinline__ V3 CtrDraw::local() {
+	const float u1 = (*this)(), u2 = (*this)();
+	return hemisphere_local(u1, u2);
+}
+struct Frame {
+	V3 n, t, b;
+};
+__device__ __forceinline__ Frame hemisphere_frame(V3 n) {
+	const V3 up = fabsf(n.z) < 0.99f ? mk(0, 0, 1) : mk(1, 0, 0);
+	const V3 t = normalize(cross(up, n));
+	return {n, t, cross(n, t)};
+}
+__device__ __forceinline__ V3 hemisphere_direction(const Frame &f, V3 local) {
+	return normalize(f.t * local.x + f.b * local.y + f.n * local.z);
 }
 
-// tracePath (src/BDPT.cpp:43-61). code (may be null) receives 2 * triangle + 1 if
-// faceViewer flipped the normal.
-template <bool kAlone, class D>
-__device__ int gi_subpath(Ctx &c, V3 o, V3 d, V3 beta, GV *out, int *code, D &draw) {
+// tracePath (src/BDPT.cpp:43-61): the path's vertices, position and 2 * triangle + 1 if
+// faceViewer flipped the normal (the throughputs follow from the triangles, see replay).
+template <class D> __device__ int gi_subpath(Ctx &c, V3 o, V3 d, float4 *out, D &draw) {
 	int k = 0;
-	for (int depth = 0; depth < kGiMaxDepth; depth++) {
-		const Hit h = kAlone ? intersect_alone(c, o, d) : intersect(c, o, d, -1);
+	for (; k < kGiMaxDepth; k++) {
+		const Hit h = intersect(c, o, d, -1);
 		if (!h.hit)
 			break;
 		const V3 tn = tri_normal(c.ref_shade, h.idx);
 		const bool flip = !(dot(tn, d) < 0.0f); // faceViewer (src/BDPT.cpp:34-36)
-		GV v;
-		v.p = h.point;
-		v.n = flip ? -tn : tn;
-		v.albedo = tri_albedo(c.ref_shade, h.idx);
-		v.beta = beta;
-		out[k] = v;
-		if (code)
-			code[k] = 2 * h.idx + (flip ? 1 : 0);
-		k++;
-		const float u1 = draw(), u2 = draw();
-		const V3 nd = cosine_hemisphere_u(v.n, u1, u2);
-		beta = beta * v.albedo;
-		o = v.p + kGiEps * nd;
-		d = nd;
+		out[k] = make_float4(h.point.x, h.point.y, h.point.z, __int_as_float(2 * h.idx + (flip ? 1 : 0)));
+		d = hemisphere_direction(hemisphere_frame(flip ? -tn : tn), draw.local());
+		o = h.point + kGiEps * d;
 	}
 	return k;
 }
+__device__ __forceinline__ Frame triangle_frame(const float4 *ref_shade, int idx, bool flip) {
+	const V3 tn = tri_normal(ref_shade, idx);
+	return hemisphere_frame(flip ? -tn : tn);
+}
 
-// The camera and light subpaths of one sample (src/BDPT.cpp:90-108). lv[0] is the
-// point on the emitter; nl counts it.
-template <bool kAlone, class D>
-__device__ void bdpt_subpaths(Ctx &c, const GiParams &p, const GiCam &cam, int x, int y, D &draw, GV *cv, int *ccode,
-                              int &nc, GV *lv, int *lcode, int &nl) {
+// A sample's first rays (src/BDPT.cpp:90-108).
+template <class D> __device__ V3 camera_direction(const GiParams &p, const GiCam &cam, int x, int y, D &draw) {
 	// glm::vec3((x + U - W/2) / f, -(y + U - H/2) / f, -1): GCC evaluates the two
 	// random arguments right to left, so the y jitter is drawn first.
 	const float uy = draw(), ux = draw();
 	const float sx = (static_cast<float>(x) + ux - static_cast<float>(p.width) / 2.0f) / p.f;
 	const float sy = -(static_cast<float>(y) + uy - static_cast<float>(p.height) / 2.0f) / p.f;
-	const V3 dir = normalize(cam.right * sx + cam.up * sy + cam.fwd * -1.0f);
-	nc = gi_subpath<kAlone>(c, cam.pos, dir, mk(1.0f, 1.0f, 1.0f), cv, ccode, draw);
+	return normalize(cam.right * sx + cam.up * sy + cam.fwd * -1.0f);
+}
+template <class D> __device__ V3 emitter_point(D &draw) {
 	const float lz = draw(), lx = draw(); // right to left again
-	const V3 lp =
-	    mk(0.0f, 0.33f, 0.0f) + mk((lx * 2.0f - 1.0f) * kGiLightHalf, 0.0f, (lz * 2.0f - 1.0f) * kGiLightHalf);
-	const V3 ln = mk(0.0f, -1.0f, 0.0f);
-	const V3 le = mk(30.0f, 30.0f, 30.0f) * gi_light_area();
-	lv[0] = GV{lp, ln, mk(0.0f, 0.0f, 0.0f), le};
-	const float d1 = draw(), d2 = draw();
-	const V3 ldir = cosine_hemisphere_u(ln, d1, d2);
-	nl = 1 + gi_subpath<kAlone>(c, lp + kGiEps * ldir, ldir, le, lv + 1, lcode, draw);
+	return mk(0.0f, 0.33f, 0.0f) + mk((lx * 2.0f - 1.0f) * kGiLightHalf, 0.0f, (lz * 2.0f - 1.0f) * kGiLightHalf);
+}
+// Both subpaths as kBdptRecordSlots vertices: the camera's from slot 0 on, the point on the
+// emitter in slot 4 and the light's vertices after it. Returns the two lengths (hits), the
+// camera's in the low four bits.
+template <class D>
+__device__ int bdpt_subpaths(Ctx &c, const GiParams &p, const GiCam &cam, int x, int y, D &draw, float4 *v) {
+	const V3 dir = camera_direction(p, cam, x, y, draw);
+	const int nc = gi_subpath(c, cam.pos, dir, v, draw);
+	const V3 lp = emitter_point(draw);
+	v[kGiMaxDepth] = make_float4(lp.x, lp.y, lp.z, 0.0f);
+	const V3 ldir = hemisphere_direction(hemisphere_frame(mk(0.0f, -1.0f, 0.0f)), draw.local());
+	return nc | (gi_subpath(c, lp + kGiEps * ldir, ldir, v + kGiMaxDepth + 1, draw) << 4);
+}
+constexpr int kBdptMinDraws = 6;                                  // a sample that hits nothing
+constexpr int kBdptMaxDraws = kBdptMinDraws + 4 * kGiMaxDepth;    // both subpaths of full length
+
+__device__ __forceinline__ void write_record(const float4 *v, int lengths, float4 *__restrict__ rec,
+                                             uint8_t *__restrict__ cnt, size_t sample) {
+	float4 *r = rec + sample * kBdptRecordSlots;
+	const int nc = lengths & 15, nl = lengths >> 4;
+	for (int i = 0; i < nc; i++)
+		r[i] = v[i];
+	for (int j = 0; j <= nl; j++)
+		r[kGiMaxDepth + j] = v[kGiMaxDepth + j];
+	cnt[sample] = static_cast<uint8_t>(lengths);
 }
 
 // Reinhard and the 8-bit pack (src/BDPT.cpp:137-141, src/Metropolis.cpp:185-189).
@@ -201,58 +189,306 @@ __device__ __forceinline__ void gi_store(const GiParams &p, long pix, V3 col, ui
 	}
 }
 
-__global__ void k_mt_seed_rows(uint32_t *s, int *idx, int rows) {
+// ---- row streams ----
+// A row's std::mt19937(9871 + y): the engine's latest generation of 624 words and a ring
+// of the outputs made but not yet consumed, as numbers in [0, 1).
+constexpr int kRing = 2048;
+struct RowStreams {
+	uint32_t *gen; // 624 words per row
+	float *ring;   // kRing per row, the unread outputs from index 0 on
+	int *unread;   // per row
+};
+
+__global__ void k_mt_seed_rows(RowStreams rs, int rows) {
 	const int y = blockIdx.x * blockDim.x + threadIdx.x;
 	if (y >= rows)
 		return;
-	uint32_t *row = s + 624 * static_cast<size_t>(y);
+	uint32_t *row = rs.gen + 624 * static_cast<size_t>(y);
 	uint32_t v = 9871u + static_cast<uint32_t>(y);
 	row[0] = v;
 	for (int k = 1; k < 624; k++) {
 		v = 1812433253u * (v ^ (v >> 30)) + static_cast<uint32_t>(k);
 		row[k] = v;
 	}
-	idx[y] = 624;
+	rs.unread[y] = 0;
 }
 
-// Traces one sample's subpaths and records them: camera vertices in slots 0-3,
-// the emitter point in slot 4, light vertices in slots 5-8 (16 B each: position
-// and 2 * triangle + normal flip), and the two lengths in cnt.
-template <bool kAlone, class D>
-__device__ __forceinline__ void record_sample(Ctx &c, const GiParams &p, const GiCam &cam, int x, int y, D &draw,
-                                              float4 *__restrict__ rec, uint8_t *__restrict__ cnt, size_t sample) {
-	GV cv[kGiMaxDepth], lv[kGiMaxDepth + 1];
-	int cc[kGiMaxDepth], lc[kGiMaxDepth], nc, nl;
-	bdpt_subpaths<kAlone>(c, p, cam, x, y, draw, cv, cc, nc, lv, lc, nl);
-	float4 *r = rec + sample * kBdptRecordSlots;
-	for (int i = 0; i < nc; i++)
-		r[i] = make_float4(cv[i].p.x, cv[i].p.y, cv[i].p.z, __int_as_float(cc[i]));
-	r[kGiMaxDepth] = make_float4(lv[0].p.x, lv[0].p.y, lv[0].p.z, 0.0f);
-	for (int j = 1; j < nl; j++)
-		r[kGiMaxDepth + j] = make_float4(lv[j].p.x, lv[j].p.y, lv[j].p.z, __int_as_float(lc[j - 1]));
-	cnt[sample] = static_cast<uint8_t>(nc | ((nl - 1) << 4));
+__device__ __forceinline__ uint32_t mt_next(uint32_t a, uint32_t b, uint32_t far) {
+	const uint32_t y = (a & 0x80000000u) | (b & 0x7fffffffu);
+	return far ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
+}
+__device__ __forceinline__ float mt_output(uint32_t y) {
+	y ^= y >> 11;
+	y ^= (y << 7) & 0x9d2c5680u;
+	y ^= (y << 15) & 0xefc60000u;
+	y ^= y >> 18;
+	return canonical01(y);
 }
 
-// Stream-order pass over columns [x0, x1): one thread per row.
-__global__ void __launch_bounds__(32) k_bdpt_rows(SceneView sv, const float4 *__restrict__ ref_shade, GiParams p,
-                                                  uint32_t *mt_s, int *mt_i, int x0, int x1,
-                                                  float4 *__restrict__ rec, uint8_t *__restrict__ cnt, int *status) {
-	if (threadIdx.x >= kRowsPerBlock)
-		return;
-	const int y = blockIdx.x * kRowsPerBlock + threadIdx.x;
-	if (y >= p.height)
-		return;
-	Ctx c{sv, ref_shade, nullptr, 0};
-	const GiCam cam = gi_cam(p);
-	MtRow rng{mt_s + 624 * static_cast<size_t>(y), mt_i[y]};
-	const int cw = x1 - x0;
-	for (int x = x0; x < x1; x++) {
-		for (int s = 0; s < p.samples; s++) {
-			const size_t sample = (static_cast<size_t>(y) * cw + (x - x0)) * p.samples + s;
-			record_sample<true>(c, p, cam, x, y, rng, rec, cnt, sample);
+// A row's stream in shared memory, advanced by a block of kT threads: the ring of outputs,
+// and beside each pair of them (every value a sample draws comes in such a pair) the
+// hemisphere coordinates it stands for, so the double-precision sine and cosine are
+// formed once per pair and not in the paths.
+template <int kT> struct RowStream {
+	uint32_t gen[2][624];
+	float ring[kRing];
+	float local[3][kRing / 2];
+	__device__ void make_locals(int from, int to) {
+		for (int i = from / 2 + threadIdx.x; i < to / 2; i += kT) {
+			const int j = i & (kRing / 2 - 1);
+			const V3 l = hemisphere_local(ring[2 * j], ring[2 * j + 1]);
+			local[0][j] = l.x;
+			local[1][j] = l.y;
+			local[2][j] = l.z;
 		}
 	}
-	mt_i[y] = rng.i;
+	__device__ void restore(const RowStreams &rs, int y, int unread) {
+		for (int i = threadIdx.x; i < 624; i += kT)
+			gen[0][i] = rs.gen[624 * static_cast<size_t>(y) + i];
+		for (int i = threadIdx.x; i < unread; i += kT)
+			ring[i] = rs.ring[kRing * static_cast<size_t>(y) + i];
+		__syncthreads();
+		make_locals(0, unread);
+		__syncthreads();
+	}
+	// The next 624 outputs, at position `made` on; cur is the latest generation. Words
+	// 227 apart depend on each other and belong to one thread.
+	__device__ void advance(int &cur, int &made) {
+		const uint32_t *s = gen[cur];
+		uint32_t *d = gen[cur ^ 1];
+		for (int t = threadIdx.x; t < 227; t += kT) {
+			const uint32_t w0 = mt_next(s[t], s[t + 1], s[t + 397]);
+			const uint32_t w1 = mt_next(s[t + 227], s[t + 228], w0);
+			d[t] = w0;
+			d[t + 227] = w1;
+			ring[(made + t) & (kRing - 1)] = mt_output(w0);
+			ring[(made + t + 227) & (kRing - 1)] = mt_output(w1);
+			const int i = t + 454;
+			if (i < 624) {
+				const uint32_t after = i < 623 ? s[i + 1] : mt_next(s[0], s[1], s[397]);
+				const uint32_t w2 = mt_next(s[i], after, w1);
+				d[i] = w2;
+				ring[(made + i) & (kRing - 1)] = mt_output(w2);
+			}
+		}
+		__syncthreads();
+		make_locals(made, made + 624);
+		made += 624;
+		cur ^= 1;
+		__syncthreads();
+	}
+	__device__ void save(const RowStreams &rs, int y, int cur, int read, int made) {
+		for (int i = threadIdx.x; i < 624; i += kT)
+			rs.gen[624 * static_cast<size_t>(y) + i] = gen[cur][i];
+		for (int i = threadIdx.x; i < made - read; i += kT)
+			rs.ring[kRing * static_cast<size_t>(y) + i] = ring[(read + i) & (kRing - 1)];
+		if (threadIdx.x == 0)
+			rs.unread[y] = made - read;
+	}
+};
+
+template <int kT> struct RingDraw {
+	const RowStream<kT> &rs;
+	int at;
+	__device__ __forceinline__ float operator()() { return rs.ring[at++ & (kRing - 1)]; }
+	__device__ __forceinline__ V3 local() {
+		const int j = (at >> 1) & (kRing / 2 - 1);
+		at += 2;
+		return mk(rs.local[0][j], rs.local[1][j], rs.local[2][j]);
+	}
+};
+
+// Stream-order pass over columns [x0, x1) of a scene with a triangle list: a block per row,
+// whose kPaths groups of kLanes lanes each follow one path (trace_closest_group). A sample's
+// light subpath starts 2 + 2 n draws after its camera subpath, whose length n is 0 to 4:
+// group 0 traces the camera subpath while the others trace the light subpaths that follow
+// the lengths most frequent of late; where none of them was right, group 1 traces the one
+// that is. The chain of rays bounds the kernel: a lone thread per row took 6 000 cycles a
+// ray, these take some 1 500 a step.
+// 640 x 480 x 16 samples, the 36-triangle box: 270 -> 37 ms.
+template <int kLanes, int kPaths>
+__global__ void __launch_bounds__(kLanes *kPaths) k_bdpt_rows_list(SceneView sv, const float4 *__restrict__ ref_shade,
+                                                                   GiParams p, RowStreams streams, int x0, int x1,
+                                                                   float4 *__restrict__ rec,
+                                                                   uint8_t *__restrict__ cnt, int *status) {
+	constexpr int kThreads = kLanes * kPaths;
+	static_assert(kThreads % 32 == 0 && kPaths >= 2, "whole warps");
+	__shared__ RowStream<kThreads> rs;
+	__shared__ TriList list;
+	__shared__ Frame frames[2 * kListTris]; // per triangle, as it is and flipped
+	__shared__ V3 normals[kListTris];
+	__shared__ int hits[2][kPaths];
+	const int y = blockIdx.x, path = threadIdx.x / kLanes;
+	const bool lead = threadIdx.x % kLanes == 0;
+	int made = streams.unread[y], read = 0, cur = 0, err = 0, odd = 0;
+	for (int i = threadIdx.x; i < 2 * sv.n_tris; i += kThreads) {
+		frames[i] = triangle_frame(ref_shade, i >> 1, (i & 1) != 0);
+		normals[i >> 1] = tri_normal(ref_shade, i >> 1);
+	}
+	list.load(sv);
+	rs.restore(streams, y, made);
+	const GiCam cam = gi_cam(p);
+	const Frame down = hemisphere_frame(mk(0.0f, -1.0f, 0.0f)); // the emitter's
+	int often[1 + kGiMaxDepth] = {}; // how often of late the camera subpath had that length
+	for (int x = x0; x < x1; x++) {
+		for (int s = 0; s < p.samples; s++) {
+			if (made - read < kBdptMaxDraws) // the same in every thread
+				rs.advance(cur, made);
+			// light path i assumes the i-th most frequent length (the same in every thread)
+			int guess = -1, nc = -1, nl = -1;
+			if (path > 0) {
+#pragma unroll
+				for (int n = 0; n <= kGiMaxDepth; n++) {
+					int before = 0;
+#pragma unroll
+					for (int m = 0; m <= kGiMaxDepth; m++)
+						before += often[m] > often[n] || (often[m] == often[n] && m > n) ? 1 : 0;
+					guess = before == path - 1 ? n : guess;
+				}
+			}
+			bool mine = path > 0; // trace a light subpath
+			float4 v[kGiMaxDepth];
+			V3 lp = mk(0.0f, 0.0f, 0.0f);
+			int n = 0;
+			for (int round = 0; nl < 0; round++) { // a second one only where no guess was right
+				RingDraw<kThreads> draw{rs, read + (mine ? 2 + 2 * guess : 0)};
+				V3 o, d;
+				if (mine) {
+					lp = emitter_point(draw);
+					d = hemisphere_direction(down, draw.local());
+					o = lp + kGiEps * d;
+				} else {
+					d = camera_direction(p, cam, x, y, draw);
+					o = cam.pos;
+				}
+				bool alive = round == 0 || mine;
+				int k = 0;
+				for (; k < kGiMaxDepth; k++) { // gi_subpath, every lane in step
+					const RayPre r = make_ray(o.x, o.y, o.z, d.x, d.y, d.z);
+					const HitRec h = trace_closest_group<kLanes>(sv, list, r, -1, err);
+					alive = alive && h.idx >= 0;
+					if (alive) {
+						const V3 point = o + h.t * d;
+						const bool flip = !(dot(normals[h.idx], d) < 0.0f); // faceViewer (src/BDPT.cpp:34-36)
+						v[k] = make_float4(point.x, point.y, point.z, __int_as_float(2 * h.idx + (flip ? 1 : 0)));
+						n = k + 1;
+						d = hemisphere_direction(frames[2 * h.idx + (flip ? 1 : 0)], draw.local());
+						o = point + kGiEps * d;
+					}
+					if (!__any_sync(0xffffffffu, alive))
+						break;
+				}
+				if (lead)
+					hits[odd][path] = mine ? n | guess << 4 : path == 0 ? n : -1;
+				__syncthreads(); // the next round writes the other row of hits
+				if (round == 0)
+					nc = hits[odd][0];
+#pragma unroll
+				for (int i = 1; i < kPaths; i++)
+					if (hits[odd][i] >> 4 == nc)
+						nl = hits[odd][i] & 15;
+				odd ^= 1;
+				if (nl < 0) {
+					mine = path == 1;
+					guess = path == 1 ? nc : -1;
+					if (mine)
+						n = 0;
+				}
+			}
+#pragma unroll
+			for (int m = 0; m <= kGiMaxDepth; m++)
+				often[m] += (m == nc ? 256 : 0) - (often[m] >> 4);
+			read += kBdptMinDraws + 2 * (nc + nl);
+			if (lead && (path == 0 || (mine && guess == nc))) {
+				const size_t sample = (static_cast<size_t>(y) * (x1 - x0) + (x - x0)) * p.samples + s;
+				float4 *r = rec + sample * kBdptRecordSlots;
+				if (path == 0) {
+					cnt[sample] = static_cast<uint8_t>(nc | (nl << 4));
+				} else {
+					r[kGiMaxDepth] = make_float4(lp.x, lp.y, lp.z, 0.0f);
+					r += kGiMaxDepth + 1;
+				}
+				for (int i = 0; i < n; i++)
+					r[i] = v[i];
+			}
+		}
+	}
+	__syncthreads();
+	rs.save(streams, y, cur, read, made);
+	if (err)
+		atomicOr(status, 1);
+}
+
+// The same for larger scenes: a block per row, kT starts on every kStride-th of its lanes.
+// Every sample takes an even number of draws, 6 to 22, so lane t traces the sample that
+// starts 2 t draws ahead, for the pixel it would most likely belong to (by the row's mean
+// draws per sample of late); thread 0 then follows the chain of starts from 0 on, as far as
+// the assumed pixels are right and the window goes, and the lanes on the chain write their
+// records. Some nine starts are traced for one that is taken, but kT lanes work in place of
+// one.
+template <int kT, int kStride>
+__global__ void __launch_bounds__(kT *kStride, 1) k_bdpt_rows(SceneView sv, const float4 *__restrict__ ref_shade, GiParams p,
+                                                  RowStreams streams, int x0, int x1, float4 *__restrict__ rec,
+                                                  uint8_t *__restrict__ cnt, int *status) {
+	static_assert(2 * kT + kBdptMaxDraws + 624 <= kRing, "the ring holds a window and a generation");
+	__shared__ RowStream<kT * kStride> rs;
+	__shared__ int next[kT], pixel[kT], slot[kT]; // per start: the draws it takes, its assumed column; its sample or -1
+	__shared__ int now[5]; // draws read, column, samples done there; draws and samples of late, for their mean
+	const int y = blockIdx.x, t = threadIdx.x / kStride;
+	const bool start = threadIdx.x % kStride == 0;
+	int made = streams.unread[y], cur = 0;
+	if (threadIdx.x == 0) {
+		now[0] = now[2] = now[3] = now[4] = 0;
+		now[1] = x0;
+	}
+	rs.restore(streams, y, made);
+	Ctx c{sv, ref_shade, nullptr, 0};
+	const GiCam cam = gi_cam(p);
+	for (;;) {
+		const int read = now[0], x = now[1], done = now[2];
+		if (x >= x1)
+			break;
+		while (made - read < 2 * kT + kBdptMaxDraws) // the same for every thread of the block
+			rs.advance(cur, made);
+		// mean draws per sample of late; before any is known, a little under the maximum
+		const float mean = now[4] > 0 ? static_cast<float>(now[3]) / static_cast<float>(now[4]) : 18.0f;
+		const int ahead = static_cast<int>(static_cast<float>(2 * t) / mean + 0.5f);
+		const int px = x + static_cast<int>((static_cast<long long>(done) + ahead) / p.samples);
+		float4 v[kBdptRecordSlots];
+		int lengths = 0;
+		if (start && px < x1) {
+			RingDraw<kT * kStride> draw{rs, read + 2 * t};
+			lengths = bdpt_subpaths(c, p, cam, px, y, draw, v);
+		}
+		if (start) {
+			next[t] = kBdptMinDraws + 2 * ((lengths & 15) + (lengths >> 4));
+			pixel[t] = px;
+			slot[t] = -1;
+		}
+		__syncthreads();
+		if (threadIdx.x == 0) {
+			int o = 0, cx = x, cs = done, n = 0;
+			while (o < 2 * kT && cx < x1 && pixel[o >> 1] == cx) {
+				slot[o >> 1] = (cx - x0) * p.samples + cs;
+				o += next[o >> 1];
+				n++;
+				if (++cs == p.samples) {
+					cs = 0;
+					cx++;
+				}
+			}
+			now[0] = read + o;
+			now[1] = cx;
+			now[2] = cs;
+			const int keep = now[4] > 2 * kT / kBdptMaxDraws ? 1 : 0; // halves what is past once it outweighs a window
+			now[3] = (now[3] >> keep) + o;
+			now[4] = (now[4] >> keep) + n;
+		}
+		__syncthreads();
+		if (start && slot[t] >= 0)
+			write_record(v, lengths, rec, cnt, static_cast<size_t>(y) * (x1 - x0) * p.samples + slot[t]);
+	}
+	rs.save(streams, y, cur, now[0], made);
 	if (c.err)
 		atomicOr(status, 1);
 }
@@ -274,7 +510,9 @@ __global__ void __launch_bounds__(128) k_bdpt_counter_paths(SceneView sv, const 
 	Ctx c{sv, ref_shade, nullptr, 0};
 	CtrDraw d{static_cast<uint32_t>(pix), static_cast<uint32_t>(s), 0u, static_cast<uint32_t>(p.seed),
 	          static_cast<uint32_t>(p.seed >> 32), 0, U4{0u, 0u, 0u, 0u}};
-	record_sample<false>(c, p, gi_cam(p), x, y, d, rec, cnt, static_cast<size_t>(i));
+	float4 v[kBdptRecordSlots];
+	const int lengths = bdpt_subpaths(c, p, gi_cam(p), x, y, d, v);
+	write_record(v, lengths, rec, cnt, static_cast<size_t>(i));
 	if (c.err)
 		atomicOr(status, 1);
 }
@@ -713,13 +951,36 @@ int bdpt_chunk_width(const GiParams &p, size_t budget) {
 	return static_cast<int>(cw);
 }
 
+// The stream-order pass: k_bdpt_rows_list for scenes with a triangle list, else k_bdpt_rows.
+// Two warps a row leave most schedulers one warp or two at 480 rows; with fewer rows there
+// is room for four, whose three guesses are right more often (480 rows: 37.0 ms with two
+// warps, 39.7 with three, 43.6 with four; 153 rows: 1.96, 1.88, 1.80). Sixteen or eight
+// lanes a ray were slower at every number of paths (45.8 ms and more): a ray's chain gets
+// longer by more than the fewer warps give back.
+// k_bdpt_rows: with one or two samples a pixel, the assumed pixels are wrong sooner, so
+// half the starts are traced, each on four times the lanes' room (an 82 000-triangle
+// sphere, 278 x 271 x 2: <64, 4> 31.2 ms, <128, 1> 36.4, one thread a row 39.5; 1 300
+// triangles, 500 x 450 x 4: 91.9, 58.4 and 91.3 ms).
+void launch_rows(const SceneView &sv, const float4 *ref_shade, const GiParams &p, const RowStreams &rs, int x0, int x1,
+                 float4 *rec, uint8_t *cnt, int *status, cudaStream_t st) {
+	const unsigned rows = static_cast<unsigned>(p.height);
+	if (sv.list && rows <= 2 * 148)
+		k_bdpt_rows_list<32, 4><<<rows, 128, 0, st>>>(sv, ref_shade, p, rs, x0, x1, rec, cnt, status);
+	else if (sv.list)
+		k_bdpt_rows_list<32, 2><<<rows, 64, 0, st>>>(sv, ref_shade, p, rs, x0, x1, rec, cnt, status);
+	else if (p.samples <= 2)
+		k_bdpt_rows<64, 4><<<rows, 256, 0, st>>>(sv, ref_shade, p, rs, x0, x1, rec, cnt, status);
+	else
+		k_bdpt_rows<128, 1><<<rows, 128, 0, st>>>(sv, ref_shade, p, rs, x0, x1, rec, cnt, status);
+}
+
 } // namespace
 
 size_t bdpt_scratch_bytes(const GiParams &p, bool reference_stream, size_t chunk_budget) {
 	(void)reference_stream; // both streams record subpaths; the row streams' state is small
 	const size_t rows = static_cast<size_t>(p.height);
 	const size_t samples = static_cast<size_t>(bdpt_chunk_width(p, chunk_budget)) * rows * p.samples;
-	return align256(624 * 4 * rows) + align256(4 * rows) + align256(samples * kBdptRecordSlots * 16) +
+	return align256(624 * 4 * rows) + align256(kRing * 4 * rows) + align256(4 * rows) + align256(samples * kBdptRecordSlots * 16) +
 	       align256(samples) + align256(samples * 4) + align256(samples * kBdptPairs * 4) +
 	       align256(samples * kBdptPairs) + 256;
 }
@@ -730,9 +991,12 @@ cudaError_t launch_bdpt(const SceneView &sv, const float4 *ref_shade, const GiPa
 	const int cw = bdpt_chunk_width(p, chunk_budget);
 	const size_t samples = static_cast<size_t>(cw) * rows * p.samples;
 	char *base = static_cast<char *>(scratch);
-	uint32_t *mt_s = reinterpret_cast<uint32_t *>(base);
+	RowStreams rs;
+	rs.gen = reinterpret_cast<uint32_t *>(base);
 	base += align256(624 * 4 * rows);
-	int *mt_i = reinterpret_cast<int *>(base);
+	rs.ring = reinterpret_cast<float *>(base);
+	base += align256(kRing * 4 * rows);
+	rs.unread = reinterpret_cast<int *>(base);
 	base += align256(4 * rows);
 	float4 *rec = reinterpret_cast<float4 *>(base);
 	base += align256(samples * kBdptRecordSlots * 16);
@@ -747,13 +1011,12 @@ cudaError_t launch_bdpt(const SceneView &sv, const float4 *ref_shade, const GiPa
 	base += align256(samples * kBdptPairs);
 	cv.count = reinterpret_cast<unsigned *>(base);
 	if (reference_stream)
-		k_mt_seed_rows<<<static_cast<unsigned>((rows + 127) / 128), 128, 0, st>>>(mt_s, mt_i, p.height);
+		k_mt_seed_rows<<<static_cast<unsigned>((rows + 127) / 128), 128, 0, st>>>(rs, p.height);
 	for (int x0 = 0; x0 < p.width; x0 += cw) {
 		const int x1 = std::min(p.width, x0 + cw);
 		if (reference_stream) {
 			TraceRange r("subpaths in row-stream order");
-			k_bdpt_rows<<<static_cast<unsigned>((rows + kRowsPerBlock - 1) / kRowsPerBlock), 32, 0, st>>>(
-			    sv, ref_shade, p, mt_s, mt_i, x0, x1, rec, cnt, status);
+			launch_rows(sv, ref_shade, p, rs, x0, x1, rec, cnt, status, st);
 		} else {
 			TraceRange r("subpaths, one thread per sample");
 			const long n = static_cast<long>(x1 - x0) * p.height * p.samples;

@@ -515,6 +515,35 @@ void flatten_bvh4(const Bvh2 &bvh, DeviceLayout4 &out) {
 	out.root_ref = 0;
 }
 
+void list_triangles(const TriangleSet &ts, const Bvh2 &bvh, std::vector<F4> &out) {
+	out.clear();
+	if (bvh.root < 0 || ts.size() > static_cast<size_t>(kMaxListTris))
+		return;
+	std::vector<int> st{bvh.root};
+	while (!st.empty()) {
+		const BvhNode &nd = bvh.nodes[static_cast<size_t>(st.back())];
+		st.pop_back();
+		if (nd.count == 0) {
+			st.push_back(nd.left);
+			st.push_back(nd.right);
+			continue;
+		}
+		for (int p = nd.start; p < nd.start + nd.count; p++) {
+			const int ti = bvh.order[static_cast<size_t>(p)];
+			const float *t = &ts.v[9 * static_cast<size_t>(ti)];
+			F4 a{t[0], t[1], t[2], 0.0f};
+			std::memcpy(&a.w, &ti, 4);
+			out.push_back(a);
+			const float e0[3] = {t[3] - t[0], t[4] - t[1], t[5] - t[2]}, e1[3] = {t[6] - t[0], t[7] - t[1], t[8] - t[2]};
+			out.push_back({e0[0], e0[1], e0[2], nd.bmin.x});
+			out.push_back({e1[0], e1[1], e1[2], nd.bmin.y});
+			out.push_back({nd.bmin.z, nd.bmax.x, nd.bmax.y, nd.bmax.z});
+			const float m[6] = {e0[1] * e1[2], e1[1] * e0[2], e0[0] * e1[2], e1[0] * e0[2], e0[0] * e1[1], e1[0] * e0[1]};
+			out.push_back({m[0] - m[1], -(m[2] - m[3]), m[4] - m[5], 0.0f});
+		}
+	}
+}
+
 void flatten_bvh(const TriangleSet &ts, const Bvh2 &bvh, DeviceLayout &out) {
 	const int n = static_cast<int>(ts.size());
 	out.nodes.clear();

@@ -122,4 +122,11 @@ struct DeviceLayout4 {
 };
 void flatten_bvh4(const Bvh2 &bvh, DeviceLayout4 &out);
 
+// The triangles of a small scene in the static traversal order, each with its leaf's box and
+// the cofactors of its edges, rounded as the triangle test rounds them: (v0, index),
+// (e0, lo.x), (e1, lo.y), (lo.z, hi.x, hi.y, hi.z), (e0.y e1.z - e1.y e0.z,
+// -(e0.x e1.z - e1.x e0.z), e0.x e1.y - e1.x e0.y, 0). Empty above kMaxListTris.
+constexpr int kMaxListTris = 128;
+void list_triangles(const TriangleSet &ts, const Bvh2 &bvh, std::vector<F4> &out);
+
 } // namespace rnb

@@ -132,9 +132,12 @@ rn_status prepare_scene(rn_scene *s) {
 	};
 	DeviceLayout4 lay4;
 	flatten_bvh4(s->bvh, lay4);
+	std::vector<F4> list;
+	list_triangles(s->tris, s->bvh, list);
 	RNB_CUDA(up(s->d_nodes, lay.nodes.data(), lay.nodes.size() * sizeof(F4)));
 	RNB_CUDA(up(s->d_nodes4, lay4.nodes.data(), lay4.nodes.size() * sizeof(F4)));
 	RNB_CUDA(up(s->d_tris, lay.tris.data(), lay.tris.size() * sizeof(F4)));
+	RNB_CUDA(up(s->d_list, list.data(), list.size() * sizeof(F4)));
 	RNB_CUDA(up(s->d_ref_shade, ref.data(), ref.size() * sizeof(F4)));
 	RNB_CUDA(up(s->d_phys_shade, phys.data(), phys.size() * sizeof(F4)));
 	RNB_CUDA(up(s->d_emitters, em.data(), em.size() * sizeof(F4)));
@@ -162,6 +165,7 @@ rn_status prepare_scene(rn_scene *s) {
 			edge = std::max({edge, std::fabs(static_cast<double>(t[3]) - t[0]), std::fabs(static_cast<double>(t[6]) - t[0])});
 		}
 	v.max_dir = edge > 0.0 ? static_cast<float>(std::min(3.0e38, std::ldexp(1.0, 123) / (edge * edge))) : 3.0e38f;
+	v.list = list.empty() ? nullptr : s->d_list.as<float4>();
 	s->view = v;
 	s->prepared = true;
 	return RN_OK;
@@ -497,8 +501,10 @@ static rn_status query_view(rn_scene *scene, unsigned flags, const char *what, S
 		view = scene->lbvh_view;
 		order = kOrderNearest;
 	}
-	if (flags & RN_PT_WIDTH2)
+	if (flags & RN_PT_WIDTH2) {
 		view.nodes4 = nullptr;
+		view.list = nullptr;
+	}
 	return RN_OK;
 }
 

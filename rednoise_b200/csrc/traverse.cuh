@@ -44,6 +44,10 @@ struct SceneView {
 	int n_tris;
 	int n_nodes;  // internal nodes of the 2-wide layout
 	int n_nodes4; // nodes of the 4-wide layout (0 when absent)
+	// Scenes of at most kListTris triangles: the triangles in the reference's static
+	// traversal order, 5 float4 each: (v0, index), (e0, leaf lo.x), (e1, leaf lo.y),
+	// (leaf lo.z, leaf hi), the cofactors of (e0, e1). Null for larger scenes.
+	const float4 *__restrict__ list;
 	// |det| <= 6 max|d| max|e|^2 in the triangle test: directions with components below
 	// max_dir keep it under 2^126
 	float max_dir;
@@ -486,7 +490,7 @@ __device__ __forceinline__ bool finite_inverse(const RayPre &r) {
 	const float inf = __int_as_float(0x7f800000);
 	return (fabsf(r.ix) < inf) & (fabsf(r.iy) < inf) & (fabsf(r.iz) < inf);
 }
-// Rays for the 4-wide tree: a finite inverse direction, and a direction
+// Rays for the 4-wide tree and the triangle list: a finite inverse direction, and a direction
 // short enough that no determinant leaves rcp_bounded's range (SceneView::max_dir).
 __device__ __forceinline__ bool bounded_ray(const SceneView &s, const RayPre &r) {
 	return finite_inverse(r) & (fmaxf(fabsf(r.dx), fmaxf(fabsf(r.dy), fabsf(r.dz))) < s.max_dir);
@@ -515,140 +519,6 @@ template <typename T, int kN> struct SharedShortStack {
 	}
 	__device__ __forceinline__ T get(int i) const { return i < kN ? col[i * stride] : spill[i - kN]; }
 };
-
-// tri_test without early exits: every quantity is formed with tri_test's
-// operations, so t, u, v and the verdict are tri_test's. Straight-line code lets a
-// thread that runs alone overlap the tests of one leaf.
-__device__ __forceinline__ bool tri_test_flat(const float4 a, const float4 b, const float4 c, const RayPre &r,
-                                              float &t, float &u, float &v) {
-	const float spx = __fsub_rn(r.ox, a.x);
-	const float spy = __fsub_rn(r.oy, a.y);
-	const float spz = __fsub_rn(r.oz, a.z);
-	const float c00 = __fsub_rn(__fmul_rn(b.y, c.z), __fmul_rn(c.y, b.z));
-	const float A = __fsub_rn(__fmul_rn(r.ndy, c.z), __fmul_rn(c.y, r.ndz));
-	const float B = __fsub_rn(__fmul_rn(r.ndy, b.z), __fmul_rn(b.y, r.ndz));
-	const float det = __fadd_rn(__fsub_rn(__fmul_rn(r.ndx, c00), __fmul_rn(b.x, A)), __fmul_rn(c.x, B));
-	const float k = __fdiv_rn(1.0f, det);
-	const float i01 = __fmul_rn(-A, k);
-	const float i11 = __fmul_rn(__fsub_rn(__fmul_rn(r.ndx, c.z), __fmul_rn(c.x, r.ndz)), k);
-	const float i21 = __fmul_rn(-__fsub_rn(__fmul_rn(r.ndx, c.y), __fmul_rn(c.x, r.ndy)), k);
-	u = __fadd_rn(__fadd_rn(__fmul_rn(i01, spx), __fmul_rn(i11, spy)), __fmul_rn(i21, spz));
-	const float i02 = __fmul_rn(B, k);
-	const float i12 = __fmul_rn(-__fsub_rn(__fmul_rn(r.ndx, b.z), __fmul_rn(b.x, r.ndz)), k);
-	const float i22 = __fmul_rn(__fsub_rn(__fmul_rn(r.ndx, b.y), __fmul_rn(b.x, r.ndy)), k);
-	v = __fadd_rn(__fadd_rn(__fmul_rn(i02, spx), __fmul_rn(i12, spy)), __fmul_rn(i22, spz));
-	const float i00 = __fmul_rn(c00, k);
-	const float i10 = __fmul_rn(-__fsub_rn(__fmul_rn(b.x, c.z), __fmul_rn(c.x, b.z)), k);
-	const float i20 = __fmul_rn(__fsub_rn(__fmul_rn(b.x, c.y), __fmul_rn(c.x, b.y)), k);
-	t = __fadd_rn(__fadd_rn(__fmul_rn(i00, spx), __fmul_rn(i10, spy)), __fmul_rn(i20, spz));
-	return !(fabsf(det) < 1e-8f) && (u >= 0.0f) && (v >= 0.0f) && (__fadd_rn(u, v) <= 1.0f) && (t > 1e-5f);
-}
-
-// Closest hit in the reference's order for a thread that runs alone: a leaf's first
-// four triangles are tested as independent straight-line work, then merged in leaf
-// order with the same strict '<'.
-template <class Stack>
-__device__ __forceinline__ HitRec trace_closest4_flat(const SceneView &s, const RayPre &r, int ignore, int &err,
-                                                      Stack &st) {
-	const RayPair r2 = make_pair_ray(r);
-	HitRec h;
-	h.idx = -1;
-	h.rank = 0x7fffffff;
-	h.t = __int_as_float(0x7f800000);
-	h.u = 0.0f;
-	h.v = 0.0f;
-	int sp = 0;
-	float te;
-	if (s.n_tris > 0 && slab(s.root_lo[0], s.root_hi[0], s.root_lo[1], s.root_hi[1], s.root_lo[2], s.root_hi[2], r, te)) {
-		st.put(0, pack_entry(s.root4_ref, te));
-		sp = 1;
-	}
-	while (sp > 0) {
-		--sp;
-		const unsigned long long e = st.get(sp);
-		int ref = static_cast<int>(static_cast<unsigned>(e));
-		if (!(__int_as_float(static_cast<int>(e >> 32)) < h.t))
-			continue;
-		while (ref >= 0) {
-			if (bad_node(s, ref, true)) {
-				err = 1;
-				return h;
-			}
-			float t[4];
-			bool b[4];
-			int4 rf;
-			node4_test(s, ref, r2, t, b, rf);
-			if (sp + 3 > kStack) {
-				err = 1;
-				return h;
-			}
-			if (b[3])
-				st.put(sp++, pack_entry(rf.w, t[3]));
-			if (b[2])
-				st.put(sp++, pack_entry(rf.z, t[2]));
-			if (b[1])
-				st.put(sp++, pack_entry(rf.y, t[1]));
-			if (b[0] && t[0] < h.t) {
-				ref = rf.x;
-			} else {
-				ref = 0x7fffffff;
-				break;
-			}
-		}
-		if (ref == 0x7fffffff)
-			continue;
-		const int start = leaf_start(ref);
-		const int count = leaf_count(ref);
-		if (bad_leaf(s, start, count)) {
-			err = 1;
-			return h;
-		}
-		if (count == 0)
-			continue;
-		float4 ta[4], tb[4], tc[4];
-#pragma unroll
-		for (int q = 0; q < 4; q++) {
-			const float4 *tp = s.tris + 3 * static_cast<size_t>(start + (q < count ? q : 0));
-			ta[q] = __ldg(tp + 0);
-			tb[q] = __ldg(tp + 1);
-			tc[q] = __ldg(tp + 2);
-		}
-		bool ok[4];
-		float tt[4], uu[4], vv[4];
-#pragma unroll
-		for (int q = 0; q < 4; q++)
-			ok[q] = tri_test_flat(ta[q], tb[q], tc[q], r, tt[q], uu[q], vv[q]) && q < count &&
-			        __float_as_int(ta[q].w) != ignore;
-#pragma unroll
-		for (int q = 0; q < 4; q++) {
-			if (ok[q] && tt[q] < h.t) {
-				h.idx = __float_as_int(ta[q].w);
-				h.t = tt[q];
-				h.u = uu[q];
-				h.v = vv[q];
-				h.rank = __float_as_int(tb[q].w);
-			}
-		}
-		for (int p = start + 4; p < start + count; p++) {
-			const float4 *tp = s.tris + 3 * static_cast<size_t>(p);
-			const float4 a = __ldg(tp + 0);
-			const int ti = __float_as_int(a.w);
-			if (ti == ignore)
-				continue;
-			const float4 b = __ldg(tp + 1);
-			const float4 c = __ldg(tp + 2);
-			float t, u, v;
-			if (tri_test(a, b, c, r, t, u, v) && t < h.t) {
-				h.idx = ti;
-				h.t = t;
-				h.u = u;
-				h.v = v;
-				h.rank = __float_as_int(b.w);
-			}
-		}
-	}
-	return h;
-}
 
 // Closest hit in the reference's order with postponed leaves (speculative traversal,
 // Aila & Laine 2009): a lane whose descent reaches a leaf keeps the leaf aside and goes on descending
@@ -782,6 +652,134 @@ __device__ __forceinline__ HitRec trace_closest4_spec(const SceneView &s, const 
 			break;
 	}
 	return h;
+}
+
+// ---- one ray by a group of lanes, for scenes of few triangles ----
+// A lone ray's traversal is a chain of dependent loads and tests: 5 000 to 20 000 cycles in
+// a scene of 36 triangles. Where rays are few, or come one after another, a group of
+// kGroup lanes takes each: every lane tests each kGroup-th triangle of the scene's list,
+// without a branch, and the group reduces to the hit.
+// The result is the reference's: a leaf's ancestors admit every ray that its own box admits
+// (rays with a finite inverse direction), so the triangles the reference may test are those
+// whose leaf's slab test passes. Of these the smallest t, the earliest in the order among
+// equals, is the hit: nothing later can replace it, and its leaf is skipped only if an
+// earlier hit lies at or before the leaf's entry distance. That distance is at most t but
+// for rounding (a wall's box is as flat as the wall); where another hit falls into the gap,
+// the exact traversal decides.
+template <int kGroup> __device__ __forceinline__ unsigned group_lanes() {
+	return kGroup == 32 ? 0xffffffffu : (1u << (kGroup % 32)) - 1u;
+}
+constexpr int kListTris = 128; // most triangles of a list (the host's kMaxListTris)
+
+// The list in shared memory, row by row, so that a group's loads are contiguous.
+struct TriList {
+	float4 row[5][kListTris];
+	__device__ __forceinline__ void load(const SceneView &s) {
+		for (int i = threadIdx.x; i < 5 * s.n_tris; i += blockDim.x)
+			row[i % 5][i / 5] = __ldg(s.list + i);
+	}
+	// Whether the leaf of triangle j is entered (te) and the triangle hit (t, u, v), with the
+	// operations of slab and tri_test and no early exit.
+	__device__ __forceinline__ bool test(int j, const RayPre &r, int ignore, float &te, float &t, float &u,
+	                                     float &v) const {
+		const float4 a = row[0][j], b = row[1][j], c = row[2][j], x = row[3][j], n = row[4][j];
+		const float t0x = __fmul_rn(__fsub_rn(b.w, r.ox), r.ix), t1x = __fmul_rn(__fsub_rn(x.y, r.ox), r.ix);
+		const float t0y = __fmul_rn(__fsub_rn(c.w, r.oy), r.iy), t1y = __fmul_rn(__fsub_rn(x.z, r.oy), r.iy);
+		const float t0z = __fmul_rn(__fsub_rn(x.x, r.oz), r.iz), t1z = __fmul_rn(__fsub_rn(x.w, r.oz), r.iz);
+		te = max3(fminf(t0x, t1x), fminf(t0y, t1y), fminf(t0z, t1z));
+		const bool in = min3(fmaxf(t0x, t1x), fmaxf(t0y, t1y), fmaxf(t0z, t1z)) >= fmaxf(te, 0.0f);
+		const float spx = __fsub_rn(r.ox, a.x), spy = __fsub_rn(r.oy, a.y), spz = __fsub_rn(r.oz, a.z);
+		const float A = __fsub_rn(__fmul_rn(r.ndy, c.z), __fmul_rn(c.y, r.ndz));
+		const float B = __fsub_rn(__fmul_rn(r.ndy, b.z), __fmul_rn(b.y, r.ndz));
+		const float det = __fadd_rn(__fsub_rn(__fmul_rn(r.ndx, n.x), __fmul_rn(b.x, A)), __fmul_rn(c.x, B));
+		const float k = rcp_bounded(det);
+		const float i01 = __fmul_rn(-A, k), i02 = __fmul_rn(B, k);
+		const float i11 = __fmul_rn(__fsub_rn(__fmul_rn(r.ndx, c.z), __fmul_rn(c.x, r.ndz)), k);
+		const float i21 = __fmul_rn(-__fsub_rn(__fmul_rn(r.ndx, c.y), __fmul_rn(c.x, r.ndy)), k);
+		const float i12 = __fmul_rn(-__fsub_rn(__fmul_rn(r.ndx, b.z), __fmul_rn(b.x, r.ndz)), k);
+		const float i22 = __fmul_rn(__fsub_rn(__fmul_rn(r.ndx, b.y), __fmul_rn(b.x, r.ndy)), k);
+		u = __fadd_rn(__fadd_rn(__fmul_rn(i01, spx), __fmul_rn(i11, spy)), __fmul_rn(i21, spz));
+		v = __fadd_rn(__fadd_rn(__fmul_rn(i02, spx), __fmul_rn(i12, spy)), __fmul_rn(i22, spz));
+		t = __fadd_rn(__fadd_rn(__fmul_rn(__fmul_rn(n.x, k), spx), __fmul_rn(__fmul_rn(n.y, k), spy)),
+		              __fmul_rn(__fmul_rn(n.z, k), spz));
+		// all of them, without a branch
+		return in & !(fabsf(det) < 1e-8f) & (u >= 0.0f) & (v >= 0.0f) & (__fadd_rn(u, v) <= 1.0f) & (t > 1e-5f) &
+		       (__float_as_int(a.w) != ignore);
+	}
+};
+
+// Closest hit of each group's ray (the same in all its lanes, which all return the hit).
+// Every lane of the warp must call it.
+template <int kGroup>
+__device__ __forceinline__ HitRec trace_closest_group(const SceneView &s, const TriList &list, const RayPre &r,
+                                                      int ignore, int &err) {
+	const int lane = threadIdx.x & 31, g = lane % kGroup, base = lane - g;
+	unsigned best_t = 0x7f800000u, best_j = 0xffffffffu; // t > 0, so its bits order as it does
+	unsigned next_t = 0x7f800000u;                       // this lane's second smallest
+	float bte = 0.0f, bu = 0.0f, bv = 0.0f;
+	for (int at = 0; at < s.n_tris; at += kGroup) { // the same number of turns in every lane
+		const int j = min(at + g, s.n_tris - 1);
+		float te, t, u, v;
+		const bool ok = list.test(j, r, ignore, te, t, u, v) & (j == at + g);
+		const unsigned bits = ok ? static_cast<unsigned>(__float_as_int(t)) : 0x7f800000u;
+		const bool better = bits < best_t;
+		next_t = min(next_t, better ? best_t : bits);
+		best_t = better ? bits : best_t;
+		best_j = better ? static_cast<unsigned>(j) : best_j;
+		bte = better ? te : bte;
+		bu = better ? u : bu;
+		bv = better ? v : bv;
+	}
+	unsigned win_t = best_t, win_j = best_j;
+	if constexpr (kGroup == 32) {
+		win_t = __reduce_min_sync(0xffffffffu, best_t);
+		win_j = __reduce_min_sync(0xffffffffu, best_t == win_t ? best_j : 0xffffffffu);
+	} else {
+#pragma unroll
+		for (int o = kGroup / 2; o > 0; o >>= 1) {
+			const unsigned ot = __shfl_xor_sync(0xffffffffu, win_t, o), oj = __shfl_xor_sync(0xffffffffu, win_j, o);
+			if (ot < win_t || (ot == win_t && oj < win_j)) {
+				win_t = ot;
+				win_j = oj;
+			}
+		}
+	}
+	const bool hit = win_t != 0x7f800000u;
+	const int from = base + static_cast<int>(win_j % kGroup);
+	const float entry = __shfl_sync(0xffffffffu, bte, from);
+	HitRec h;
+	h.t = __int_as_float(static_cast<int>(win_t));
+	h.u = __shfl_sync(0xffffffffu, bu, from);
+	h.v = __shfl_sync(0xffffffffu, bv, from);
+	h.idx = hit ? __float_as_int(list.row[0][win_j % kListTris].w) : -1;
+	h.rank = hit ? static_cast<int>(win_j) : 0x7fffffff;
+	if (!hit)
+		h.u = h.v = 0.0f;
+	// another hit, perhaps an earlier one, in the gap before the entry?
+	const unsigned other = lane == from ? next_t : best_t;
+	const bool gap = hit & (entry > h.t) & (other != 0x7f800000u) & (__int_as_float(static_cast<int>(other)) <= entry);
+	const unsigned exact = __ballot_sync(0xffffffffu, gap | !bounded_ray(s, r));
+	if (exact & (group_lanes<kGroup>() << base))
+		h = trace_closest<kOrderReference>(s, r, ignore, err);
+	return h;
+}
+
+// Occlusion of each group's ray before tmax (the order does not matter). Every lane of the
+// warp must call it.
+template <int kGroup>
+__device__ __forceinline__ bool trace_any_group(const SceneView &s, const TriList &list, const RayPre &r, float tmax,
+                                                int ignore, int &err) {
+	const int lane = threadIdx.x & 31, g = lane % kGroup;
+	bool any = false;
+	if (!bounded_ray(s, r)) {
+		any = trace_any(s, r, tmax, ignore, err);
+	} else {
+		for (int j = g; j < s.n_tris; j += kGroup) {
+			float te, t, u, v;
+			any |= list.test(j, r, ignore, te, t, u, v) & (te < tmax) & (t < tmax);
+		}
+	}
+	return (__ballot_sync(0xffffffffu, any) & (group_lanes<kGroup>() << (lane - g))) != 0;
 }
 
 // Any hit with postponed leaves (the closest-hit version's scheme): occlusion does not
