@@ -1,6 +1,7 @@
 #include "host_scene.hpp"
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -407,27 +408,37 @@ void flatten_bvh4(const Bvh2 &bvh, DeviceLayout4 &out) {
 		out.root_ref = leaf_ref(root);
 		return;
 	}
-	// Which reference levels become 4-wide nodes. Every node spans two reference
-	// levels at most, and any such frontier gives the same traversal result, so the
-	// choice only moves cost: each 4-wide node costs one fetch per ray that reaches
-	// it, about in proportion to its box's surface area. Bottom-up over the tree,
-	// F(n) = area(n) + sum over n's children c of G(c) is the cost below n when n
-	// roots a 4-wide node, and G(c) = min(F(c), F of c's internal children) picks,
-	// per internal child, between keeping it as an entry and splicing its two
-	// children in. On a complete tree of odd height this puts the 4-wide nodes at
-	// even heights above the leaves (all nodes full, about half as many) where a
-	// top-down collapse leaves the bottom level half empty.
+	// Which binary nodes become entries. Any frontier gives the same traversal result, so the
+	// choice only moves cost: each 4-wide node costs one fetch per ray that reaches it, about
+	// in proportion to its box's surface area. Bottom-up over the tree, cost[n][i] is the least
+	// cost of the 4-wide nodes below n when n is represented by at most i + 1 entries (itself,
+	// or a frontier of its descendants), and an entry that roots a 4-wide node divides four
+	// entries between its two children.
 	const size_t nn = bvh.nodes.size();
-	std::vector<double> cost_root(nn, 0.0), cost_best(nn, 0.0);
-	std::vector<char> splice(nn, 0);
+	std::vector<std::array<float, 3>> cost(nn, {0.0f, 0.0f, 0.0f});
+	auto is_leaf = [&](int i) { return bvh.nodes[static_cast<size_t>(i)].count > 0; };
+	// the cheapest way to give `entries` (2 to 4) entries to n's children: entries of the left one
+	auto divide = [&](const BvhNode &nd, int entries, float &best) {
+		int left = 1;
+		best = std::numeric_limits<float>::infinity();
+		for (int i = 1; i < entries; i++) {
+			const float c = cost[static_cast<size_t>(nd.left)][static_cast<size_t>(i - 1)] +
+			                cost[static_cast<size_t>(nd.right)][static_cast<size_t>(entries - i - 1)];
+			if (c < best || (c == best && std::abs(2 * i - entries) < std::abs(2 * left - entries))) {
+				best = c;
+				left = i;
+			}
+		}
+		return left;
+	};
 	{
 		auto area = [](const BvhNode &nd) {
-			const double x = std::max(0.0, static_cast<double>(nd.bmax.x) - nd.bmin.x);
-			const double y = std::max(0.0, static_cast<double>(nd.bmax.y) - nd.bmin.y);
-			const double z = std::max(0.0, static_cast<double>(nd.bmax.z) - nd.bmin.z);
+			const float x = std::max(0.0f, nd.bmax.x - nd.bmin.x), y = std::max(0.0f, nd.bmax.y - nd.bmin.y),
+			            z = std::max(0.0f, nd.bmax.z - nd.bmin.z);
 			return x * y + y * z + z * x;
 		};
 		std::vector<int> pre; // pre-order; walked backwards, children come before parents
+		pre.reserve(nn);
 		std::vector<int> st{bvh.root};
 		while (!st.empty()) {
 			const int i = st.back();
@@ -439,23 +450,39 @@ void flatten_bvh4(const Bvh2 &bvh, DeviceLayout4 &out) {
 				st.push_back(nd.right);
 			}
 		}
-		auto internal_root_cost = [&](int c) {
-			return bvh.nodes[static_cast<size_t>(c)].count > 0 ? 0.0 : cost_root[static_cast<size_t>(c)];
-		};
 		for (size_t k = pre.size(); k-- > 0;) {
-			const int i = pre[k];
-			const BvhNode &nd = bvh.nodes[static_cast<size_t>(i)];
+			const BvhNode &nd = bvh.nodes[static_cast<size_t>(pre[k])];
 			if (nd.count > 0)
 				continue;
-			const size_t l = static_cast<size_t>(nd.left), r = static_cast<size_t>(nd.right);
-			const bool leaf_l = bvh.nodes[l].count > 0, leaf_r = bvh.nodes[r].count > 0;
-			cost_root[static_cast<size_t>(i)] =
-			    area(nd) + (leaf_l ? 0.0 : cost_best[l]) + (leaf_r ? 0.0 : cost_best[r]);
-			const double spliced = internal_root_cost(nd.left) + internal_root_cost(nd.right);
-			splice[static_cast<size_t>(i)] = spliced < cost_root[static_cast<size_t>(i)];
-			cost_best[static_cast<size_t>(i)] = std::min(cost_root[static_cast<size_t>(i)], spliced);
+			auto &c = cost[static_cast<size_t>(pre[k])];
+			float best;
+			divide(nd, 4, best);
+			c[0] = area(nd) + best;
+			for (int e = 2; e <= 3; e++) {
+				divide(nd, e, best);
+				c[static_cast<size_t>(e - 1)] = std::min(c[static_cast<size_t>(e - 2)], best);
+			}
 		}
 	}
+	// Appends node n's entries, at most `entries` of them, in pop order (right side first).
+	struct Frontier {
+		int ent[4];
+		int cnt = 0;
+	};
+	auto expand = [&](auto &&self, int n, int entries, Frontier &f) -> void {
+		const BvhNode &nd = bvh.nodes[static_cast<size_t>(n)];
+		float best = 0.0f;
+		const auto &c = cost[static_cast<size_t>(n)];
+		while (entries > 1 && c[static_cast<size_t>(entries - 1)] == c[static_cast<size_t>(entries - 2)])
+			entries--; // as cheap with fewer
+		if (is_leaf(n) || entries == 1) {
+			f.ent[f.cnt++] = n;
+			return;
+		}
+		const int left = divide(nd, entries, best);
+		self(self, nd.right, entries - left, f);
+		self(self, nd.left, left, f);
+	};
 	// Iterative build: each work item fills node `slot` from reference node `src`.
 	std::vector<std::pair<int, int>> work; // (slot, src)
 	out.nodes.resize(8);
@@ -464,18 +491,13 @@ void flatten_bvh4(const Bvh2 &bvh, DeviceLayout4 &out) {
 		const auto [slot, src] = work.back();
 		work.pop_back();
 		const BvhNode &n = bvh.nodes[static_cast<size_t>(src)];
-		// Entries in pop order: right side first, and within a side its right child first.
-		int ent[4];
-		int cnt = 0;
-		for (int c : {n.right, n.left}) {
-			const BvhNode &cn = bvh.nodes[static_cast<size_t>(c)];
-			if (cn.count > 0 || !splice[static_cast<size_t>(c)]) {
-				ent[cnt++] = c;
-			} else {
-				ent[cnt++] = cn.right;
-				ent[cnt++] = cn.left;
-			}
-		}
+		float best = 0.0f;
+		const int left = divide(n, 4, best);
+		Frontier f;
+		expand(expand, n.right, 4 - left, f);
+		expand(expand, n.left, left, f);
+		const int cnt = f.cnt;
+		const int *ent = f.ent;
 		float lo[3][4], hi[3][4];
 		int refs[4];
 		for (int k = 0; k < 4; k++) {
@@ -542,6 +564,130 @@ void list_triangles(const TriangleSet &ts, const Bvh2 &bvh, std::vector<F4> &out
 			out.push_back({m[0] - m[1], -(m[2] - m[3]), m[4] - m[5], 0.0f});
 		}
 	}
+}
+
+int stack_need4(const DeviceLayout4 &layout) {
+	// A node pushes its entries but the first, last one first, and descends into the first
+	// (which for leaves may wait while the next is popped: one more). Children follow
+	// their parents in the node array.
+	const size_t n = layout.nodes.size() / 8;
+	if (n == 0)
+		return 1;
+	auto as_int = [](float f) {
+		int i;
+		std::memcpy(&i, &f, 4);
+		return i;
+	};
+	std::vector<int> below(n, 0); // entries on the stack when the node is reached
+	int need = 1;
+	for (size_t k = 0; k < n; k++) {
+		const F4 &r = layout.nodes[8 * k + 6];
+		const int refs[4] = {as_int(r.x), as_int(r.y), as_int(r.z), as_int(r.w)};
+		const int cnt = as_int(layout.nodes[8 * k + 7].x);
+		need = std::max(need, below[k] + 3); // what the traversals check before they push
+		for (int e = 0; e < cnt; e++)
+			if (refs[e] >= 0)
+				below[static_cast<size_t>(refs[e])] = below[k] + cnt - 1 - e;
+	}
+	return need;
+}
+
+namespace {
+
+struct AreaTree {
+	const Bvh2 &ref;
+	Bvh2 &out;
+	std::vector<int> leaves;   // reference leaves in pop order
+	std::vector<float> suffix; // scratch: areas of the boxes of [k, end)
+
+	static void grow(Vec3 &lo, Vec3 &hi, const BvhNode &n) {
+		lo = {gmin(lo.x, n.bmin.x), gmin(lo.y, n.bmin.y), gmin(lo.z, n.bmin.z)};
+		hi = {gmax(hi.x, n.bmax.x), gmax(hi.y, n.bmax.y), gmax(hi.z, n.bmax.z)};
+	}
+	static float half_area(const Vec3 &lo, const Vec3 &hi) {
+		const float x = hi.x - lo.x, y = hi.y - lo.y, z = hi.z - lo.z;
+		return x * y + y * z + z * x;
+	}
+	const BvhNode &leaf(size_t k) const { return ref.nodes[static_cast<size_t>(leaves[k])]; }
+
+	// Nodes of [i, j) go to slots self, self + 1, ... (2 (j - i) - 1 of them, in pre-order).
+	// The top par_levels levels build their first part on a thread of its own; beyond
+	// max_depth ranges are halved, so the depth stays bounded.
+	void build(size_t self, size_t i, size_t j, int depth, int par_levels) {
+		if (j - i == 1) {
+			out.nodes[self] = leaf(i);
+			return;
+		}
+		BvhNode node;
+		node.bmin = leaf(j - 1).bmin;
+		node.bmax = leaf(j - 1).bmax;
+		size_t split = i + (j - i) / 2;
+		constexpr int kMaxSahDepth = 40;
+		if (depth < kMaxSahDepth) {
+			Vec3 lo = node.bmin, hi = node.bmax;
+			for (size_t k = j - 1; k > i; k--) {
+				grow(lo, hi, leaf(k));
+				suffix[k] = half_area(lo, hi);
+			}
+			grow(lo, hi, leaf(i));
+			node.bmin = lo;
+			node.bmax = hi;
+			float best = std::numeric_limits<float>::infinity();
+			lo = leaf(i).bmin;
+			hi = leaf(i).bmax;
+			for (size_t k = i + 1; k < j; k++) {
+				const float cost = half_area(lo, hi) * static_cast<float>(k - i) + suffix[k] * static_cast<float>(j - k);
+				if (cost < best) {
+					best = cost;
+					split = k;
+				}
+				grow(lo, hi, leaf(k));
+			}
+		} else {
+			for (size_t k = i; k < j - 1; k++)
+				grow(node.bmin, node.bmax, leaf(k));
+		}
+		// the first part is popped first: the right child
+		const size_t right = self + 1, left = right + 2 * (split - i) - 1;
+		node.right = static_cast<int>(right);
+		node.left = static_cast<int>(left);
+		out.nodes[self] = node;
+		if (par_levels > 0 && j - i > 4096) {
+			std::thread first([=, this] { build(right, i, split, depth + 1, par_levels - 1); });
+			build(left, split, j, depth + 1, par_levels - 1);
+			first.join();
+		} else {
+			build(right, i, split, depth + 1, 0);
+			build(left, split, j, depth + 1, 0);
+		}
+	}
+};
+
+} // namespace
+
+void split_by_area(const Bvh2 &bvh, Bvh2 &out) {
+	out = Bvh2();
+	if (bvh.root < 0)
+		return;
+	out.order = bvh.order;
+	AreaTree t{bvh, out, {}, {}};
+	std::vector<int> st{bvh.root};
+	while (!st.empty()) {
+		const int i = st.back();
+		st.pop_back();
+		const BvhNode &nd = bvh.nodes[static_cast<size_t>(i)];
+		if (nd.count > 0) {
+			t.leaves.push_back(i);
+		} else {
+			st.push_back(nd.left);
+			st.push_back(nd.right);
+		}
+	}
+	t.suffix.resize(t.leaves.size());
+	out.nodes.resize(2 * t.leaves.size() - 1);
+	out.root = 0;
+	out.depth = bvh.depth;
+	t.build(0, 0, t.leaves.size(), 1, 6);
 }
 
 void flatten_bvh(const TriangleSet &ts, const Bvh2 &bvh, DeviceLayout &out) {

@@ -4,6 +4,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <future>
 #include <new>
 #include <string>
 
@@ -75,6 +76,20 @@ rn_status prepare_scene(rn_scene *s) {
 	int dev = 0;
 	RNB_CUDA(cudaGetDevice(&dev));
 	s->device = dev;
+	// The 4-wide tree, while this thread lays out the reference's and the shading records. A
+	// scene of few triangles keeps the reference's shape: there is little to skip above its
+	// leaves, and ranges of unequal length make its few nodes deeper.
+	auto four = std::async(std::launch::async, [s] {
+		DeviceLayout4 out;
+		if (s->tris.size() > static_cast<size_t>(kMaxListTris)) {
+			Bvh2 tree;
+			split_by_area(s->bvh, tree);
+			flatten_bvh4(tree, out);
+		}
+		if (out.nodes.empty() || stack_need4(out) > kStack) // or a tree of chains: the reference's is balanced
+			flatten_bvh4(s->bvh, out);
+		return out;
+	});
 	auto t0 = std::chrono::steady_clock::now();
 	DeviceLayout lay;
 	flatten_bvh(s->tris, s->bvh, lay);
@@ -130,8 +145,7 @@ rn_status prepare_scene(rn_scene *s) {
 			return cudaMemcpy(b.p, src, bytes, cudaMemcpyHostToDevice);
 		return cudaSuccess;
 	};
-	DeviceLayout4 lay4;
-	flatten_bvh4(s->bvh, lay4);
+	const DeviceLayout4 lay4 = four.get();
 	std::vector<F4> list;
 	list_triangles(s->tris, s->bvh, list);
 	RNB_CUDA(up(s->d_nodes, lay.nodes.data(), lay.nodes.size() * sizeof(F4)));

@@ -380,36 +380,15 @@ __device__ __forceinline__ bool trace_any(const SceneView &s, const RayPre &r, f
 }
 
 // ---- 4-wide traversal in the reference's order ---------------------------------
-// Entries of a node are stored in the order the reference pops them; entries
-// 1..count-1 are pushed (last first) and entry 0 is descended into at once,
-// which is the reference's push-then-pop. Every box is a reference node box and
-// is tested with the reference's slab arithmetic; a skipped intermediate box is
-// implied by its children's tests (monotone rounding), so closest hit and
-// occlusion equal the reference's. Rays with an infinite 1/d component (a zero
-// or subnormal direction component, where a slab product can be NaN) take the
-// 2-wide path instead.
-
-// Paired single-precision arithmetic of sm_100 (PTX add/sub/mul .rn.f32x2): two
-// independently, correctly rounded IEEE operations per instruction, so the slab
-// products keep the reference's bits at half the instruction count.
-__device__ __forceinline__ unsigned long long pair2(float lo, float hi) {
-	unsigned long long r;
-	asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-	return r;
-}
-__device__ __forceinline__ void unpair2(unsigned long long v, float &lo, float &hi) {
-	asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b) {
-	unsigned long long r;
-	asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-	return r;
-}
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
-	unsigned long long r;
-	asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-	return r;
-}
+// The tree is the host's own over the reference tree's leaves (split_by_area), which it meets in
+// the reference's order. Entries of a node are stored in that order; entries 1..count-1 are
+// pushed (last first) and entry 0 is descended into at once, which is the reference's
+// push-then-pop. The reference reaches a leaf whose own box the ray enters before the best
+// distance of that moment, for then it passed every box above it too (boxes that contain
+// the leaf's are entered no later: the slab arithmetic rounds monotonically); so do these
+// traversals, whatever boxes stand above the leaves. Rays with an infinite 1/d component (a
+// zero or subnormal direction component, where a slab product can be NaN) take the 2-wide
+// path instead.
 
 // Three-input min / max of sm_100 (PTX min.f32 / max.f32 with three sources).
 __device__ __forceinline__ float max3(float a, float b, float c) {
