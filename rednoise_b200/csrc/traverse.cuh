@@ -390,6 +390,30 @@ __device__ __forceinline__ bool trace_any(const SceneView &s, const RayPre &r, f
 // zero or subnormal direction component, where a slab product can be NaN) take the 2-wide
 // path instead.
 
+// Paired single-precision arithmetic of sm_100 (PTX sub/mul .rn.f32x2): two independently,
+// correctly rounded IEEE operations per instruction, so the slab products keep the
+// reference's bits at half the instruction count. A product may only feed scalar sums: ptxas
+// contracts mul.rn.f32x2 into a following packed sum in spite of .rn (measured), while the
+// slab's order, differences first, leaves it nothing to contract.
+__device__ __forceinline__ unsigned long long pair2(float lo, float hi) {
+	unsigned long long r;
+	asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+	return r;
+}
+__device__ __forceinline__ void unpair2(unsigned long long v, float &lo, float &hi) {
+	asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b) {
+	unsigned long long r;
+	asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+	return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+	unsigned long long r;
+	asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+	return r;
+}
+
 // Three-input min / max of sm_100 (PTX min.f32 / max.f32 with three sources).
 __device__ __forceinline__ float max3(float a, float b, float c) {
 	float r;
