@@ -39,6 +39,43 @@ __global__ void __launch_bounds__(128) k_trace_any(SceneView s, int n, const flo
 	occ[i] = hit ? 1 : 0;
 }
 
+// Many rays: a persistent grid whose lanes take the next ray when theirs is done.
+constexpr int kStreamBlocks = 7;                                    // per SM: 72 registers, what measured best
+constexpr size_t kStreamSmem = 128 * 8 * sizeof(unsigned long long); // the stacks' tops
+__global__ void __launch_bounds__(128, kStreamBlocks)
+    k_trace_closest_stream(SceneView s, int n, const float *__restrict__ o, const float *__restrict__ d,
+                           const int *__restrict__ ignore, int *__restrict__ tri, float *__restrict__ t,
+                           float *__restrict__ u, float *__restrict__ v, int *err) {
+	extern __shared__ unsigned long long closest_top[];
+	SharedShortStack<unsigned long long, 8> st(closest_top + threadIdx.x, blockDim.x);
+	StreamTurns turns(static_cast<unsigned>(n));
+	int e = 0;
+	unsigned i = 0;
+	trace_closest_stream(
+	    s, st, e,
+	    [&](bool want, unsigned idle, RayPre &r, int &ig) {
+		    unsigned k;
+		    if (!turns.next(want, idle, k))
+			    return false;
+		    i = k;
+		    const size_t a = 3 * static_cast<size_t>(i);
+		    r = make_ray(o[a], o[a + 1], o[a + 2], d[a], d[a + 1], d[a + 2]);
+		    ig = ignore ? ignore[i] : -1;
+		    return true;
+	    },
+	    [&](const HitRec &h) {
+		    tri[i] = h.idx;
+		    if (t)
+			    t[i] = h.t;
+		    if (u)
+			    u[i] = h.u;
+		    if (v)
+			    v[i] = h.v;
+	    });
+	if (e)
+		atomicOr(err, 1);
+}
+
 // Few rays over a small scene: kGroup lanes per ray (trace_closest_group).
 constexpr int kGroup = 8;
 __global__ void __launch_bounds__(128) k_trace_closest_group(SceneView s, int n, const float *__restrict__ o,
@@ -89,6 +126,10 @@ __global__ void __launch_bounds__(128) k_trace_any_group(SceneView s, int n, con
 // the 36-triangle box take 6 us of device time for 4 096 rays (39 with a thread per ray), 12
 // (40) for 16 384, 31 (45) for 65 536 and 62 (56) for 131 072.
 constexpr int kGroupRays = 1 << 16;
+// Closest hits of this many rays and more, over larger scenes, take the persistent kernel: below
+// it too few warps have a ray to go on with (65 536 rays over 1.31M triangles 180 us, 201
+// with it; 262 144 over 82 000 triangles 216 and 207; 2M over 1.31M 1 081 and 884).
+constexpr int kStreamRays = 1 << 17;
 
 cudaError_t launch_trace_closest(const SceneView &v, int n, const float *o, const float *d, const int *ignore,
                                  int order, int *tri, float *t, float *u, float *vv, int *err, cudaStream_t st) {
@@ -100,6 +141,8 @@ cudaError_t launch_trace_closest(const SceneView &v, int n, const float *o, cons
 		                                                                                  vv, err);
 	else if (order == kOrderNearest)
 		k_trace_closest<kOrderNearest><<<ceil_div(n, bs), bs, 0, st>>>(v, n, o, d, ignore, tri, t, u, vv, err);
+	else if (v.nodes4 && !v.list && n >= kStreamRays)
+		k_trace_closest_stream<<<148 * kStreamBlocks, bs, kStreamSmem, st>>>(v, n, o, d, ignore, tri, t, u, vv, err);
 	else
 		k_trace_closest<kOrderReference><<<ceil_div(n, bs), bs, 0, st>>>(v, n, o, d, ignore, tri, t, u, vv, err);
 	return cudaGetLastError();
