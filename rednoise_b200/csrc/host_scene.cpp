@@ -767,8 +767,10 @@ void flatten_bvh(const TriangleSet &ts, const Bvh2 &bvh, DeviceLayout &out) {
 		const float *t = &ts.v[9 * static_cast<size_t>(ti)];
 		F4 *o = &out.tris[3 * static_cast<size_t>(p)];
 		o[0] = {t[0], t[1], t[2], as_float(ti)};
-		o[1] = {t[3] - t[0], t[4] - t[1], t[5] - t[2], as_float(rank_of_pos[static_cast<size_t>(p)])};
-		o[2] = {t[6] - t[0], t[7] - t[1], t[8] - t[2], 0.0f};
+		const float e0[3] = {t[3] - t[0], t[4] - t[1], t[5] - t[2]}, e1[3] = {t[6] - t[0], t[7] - t[1], t[8] - t[2]};
+		const float yz = e0[1] * e1[2], zy = e1[1] * e0[2]; // rounded one by one
+		o[1] = {e1[0], e0[0], e1[1], e0[1]};
+		o[2] = {e1[2], e0[2], yz - zy, as_float(rank_of_pos[static_cast<size_t>(p)])};
 	}
 }
 

@@ -87,7 +87,8 @@ bool load_obj(const std::string &path, float scale, TriangleSet &out, std::strin
 //     n3 = (ref L, ref R, -, -) as int bits
 //  child ref >= 0: dense internal node index; ref < 0: leaf ~((start << 3) | count)
 //  tris: 3 float4 per triangle position in leaf order:
-//     (v0.xyz, original index), (e0 = v1 - v0, rank), (e1 = v2 - v0, 0)
+//     (v0.xyz, original index), (e1.x, e0.x, e1.y, e0.y),
+//     (e1.z, e0.z, e0.y * e1.z - e1.y * e0.z, rank), e0 = v1 - v0, e1 = v2 - v0
 //  rank = position of the triangle in the reference's static traversal order
 //  (leaves visited right child first, triangles ascending within a leaf).
 struct F4 {

@@ -184,12 +184,14 @@ __global__ void k_refit(const float *__restrict__ v9, const int *__restrict__ or
 		b.hi[a] = fmax3(t[a], t[3 + a], t[6 + a]);
 	}
 	leaf_box[p] = b;
-	// v0, e0 = v1 - v0, e1 = v2 - v0 (IEEE subtraction, as the host layout); rank = leaf position
+	// v0, e0 = v1 - v0, e1 = v2 - v0 and their x cofactor, laid out and rounded as the host
+	// layout's; rank = leaf position
 	tris[3 * static_cast<size_t>(p)] = make_float4(t[0], t[1], t[2], __int_as_float(ti));
-	tris[3 * static_cast<size_t>(p) + 1] =
-	    make_float4(__fsub_rn(t[3], t[0]), __fsub_rn(t[4], t[1]), __fsub_rn(t[5], t[2]), __int_as_float(p));
-	tris[3 * static_cast<size_t>(p) + 2] =
-	    make_float4(__fsub_rn(t[6], t[0]), __fsub_rn(t[7], t[1]), __fsub_rn(t[8], t[2]), 0.0f);
+	const float e0x = __fsub_rn(t[3], t[0]), e0y = __fsub_rn(t[4], t[1]), e0z = __fsub_rn(t[5], t[2]);
+	const float e1x = __fsub_rn(t[6], t[0]), e1y = __fsub_rn(t[7], t[1]), e1z = __fsub_rn(t[8], t[2]);
+	const float c00 = __fsub_rn(__fmul_rn(e0y, e1z), __fmul_rn(e1y, e0z));
+	tris[3 * static_cast<size_t>(p) + 1] = make_float4(e1x, e0x, e1y, e0y);
+	tris[3 * static_cast<size_t>(p) + 2] = make_float4(e1z, e0z, c00, __int_as_float(p));
 	if (n == 1)
 		return;
 	int node = parent_leaf[p];

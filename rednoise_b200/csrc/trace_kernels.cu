@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(128) k_trace_any_group(SceneView s, int n, con
 constexpr int kGroupRays = 1 << 16;
 // Closest hits of this many rays and more, over larger scenes, take the persistent kernel: below
 // it too few warps have a ray to go on with (65 536 rays over 1.31M triangles 180 us, 201
-// with it; 262 144 over 82 000 triangles 216 and 207; 2M over 1.31M 1 081 and 884).
+// with it; 262 144 over 82 000 triangles 216 and 207; 2M over 1.31M 1 081 and 884; now 778).
 constexpr int kStreamRays = 1 << 17;
 
 cudaError_t launch_trace_closest(const SceneView &v, int n, const float *o, const float *d, const int *ignore,

@@ -68,6 +68,30 @@ struct HitRec {
 };
 
 #ifdef __CUDACC__
+// Paired single-precision arithmetic of sm_100 (PTX sub/mul .rn.f32x2): two independently,
+// correctly rounded IEEE operations per instruction, so products keep the reference's
+// bits at half the instruction count. A product may only feed scalar sums: ptxas
+// contracts mul.rn.f32x2 into a following packed sum in spite of .rn (measured), while the
+// slab's order, differences first, leaves it nothing to contract.
+__device__ __forceinline__ unsigned long long pair2(float lo, float hi) {
+	unsigned long long r;
+	asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+	return r;
+}
+__device__ __forceinline__ void unpair2(unsigned long long v, float &lo, float &hi) {
+	asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b) {
+	unsigned long long r;
+	asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+	return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+	unsigned long long r;
+	asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+	return r;
+}
+
 __device__ __forceinline__ RayPre make_ray(float ox, float oy, float oz, float dx, float dy, float dz) {
 	RayPre r;
 	r.ox = ox;
@@ -121,43 +145,64 @@ __device__ __forceinline__ bool slab(float lox, float hix, float loy, float hiy,
 	return tx >= m0;
 }
 
-// Reference ray/triangle test on a stored (v0, e0 = v1 - v0, e1 = v2 - v0)
-// record; e0/e1 were computed on the host with the same IEEE subtraction the
+// Reference ray/triangle test on a stored record of (v0, e0 = v1 - v0, e1 = v2 - v0):
+// a = (v0, index), b = (e1.x, e0.x, e1.y, e0.y), c = (e1.z, e0.z, e0.y * e1.z - e1.y * e0.z,
+// rank). e0, e1 and the cofactor were computed on the host with the IEEE operations the
 // reference performs at test time, so they carry the same bits. kBounded: the ray is a
 // bounded_ray of the scene, whose determinants stay in rcp_bounded's range (those below
 // 1e-8 are rejected whatever their reciprocal).
-template <bool kBounded = false>
+// u needs the cofactors of e1, v those of e0, in the same expressions: the record holds the
+// edges side by side and their products are formed in pairs. (Expressions are the
+// reference's with signs moved, which changes no bit: -(x * y) and (-x) * y are the same, and so
+// are (-x) - (-y) and y - x.)
+// A ray takes 10 to 14 of these tests, with 18 to 20 of a warp's lanes in step, and a warp
+// rarely leaves at an early exit of its lanes: between the determinant and t there is one,
+// behind u and v together, and the 4-wide traversals load the whole record before they look
+// at the index to ignore. Against the reference's order of tests and unpaired products: the
+// 1.31M-triangle 1080p x 32 spp frame 47.9 -> 45.5 ms, the room at 720p x 64 spp 25.2 ->
+// 24.4, the drop-in's 320 x 240 x 16 frame 3.42 -> 3.06, four adjoint views of the room
+// 24.6 -> 22.8. kStraight has no exit at all: for rays that share nothing but the warp (2M
+// unordered ones 0.83 -> 0.78 ms), while the room's frames lose 2 % with it.
+template <bool kBounded = false, bool kStraight = false>
 __device__ __forceinline__ bool tri_test(const float4 a, const float4 b, const float4 c, const RayPre &r, float &t,
                                          float &u, float &v) {
 	const float spx = __fsub_rn(r.ox, a.x);
 	const float spy = __fsub_rn(r.oy, a.y);
 	const float spz = __fsub_rn(r.oz, a.z);
-	// mat3(m0 = -d, m1 = e0, m2 = e1); cofactors named after glm's expressions.
-	const float c00 = __fsub_rn(__fmul_rn(b.y, c.z), __fmul_rn(c.y, b.z));     // m11*m22 - m21*m12
-	const float A = __fsub_rn(__fmul_rn(-r.dy, c.z), __fmul_rn(c.y, -r.dz));   // m01*m22 - m21*m02
-	const float B = __fsub_rn(__fmul_rn(-r.dy, b.z), __fmul_rn(b.y, -r.dz));   // m01*m12 - m11*m02
-	const float det = __fadd_rn(__fsub_rn(__fmul_rn(-r.dx, c00), __fmul_rn(b.x, A)), __fmul_rn(c.x, B));
-	if (fabsf(det) < 1e-8f)
+	const unsigned long long X = pair2(b.x, b.y), Y = pair2(b.z, b.w), Z = pair2(c.x, c.y);
+	const unsigned long long dx = pair2(r.dx, r.dx), dy = pair2(r.dy, r.dy), dz = pair2(r.dz, r.dz);
+	// mat3(m0 = -d, m1 = e0, m2 = e1): A = m01*m22 - m21*m02, B = m01*m12 - m11*m02
+	float p0, p1, q0, q1;
+	unpair2(mul2(Y, dz), p0, p1);
+	unpair2(mul2(dy, Z), q0, q1);
+	const float A = __fsub_rn(p0, q0), B = __fsub_rn(p1, q1);
+	const float det = __fadd_rn(__fsub_rn(__fmul_rn(-r.dx, c.z), __fmul_rn(b.y, A)), __fmul_rn(b.x, B));
+	if (!kStraight && fabsf(det) < 1e-8f)
 		return false;
 	const float k = kBounded ? rcp_bounded(det) : __fdiv_rn(1.0f, det);
-	// Row 1 of the inverse gives u.
-	const float i01 = __fmul_rn(-A, k);
-	const float i11 = __fmul_rn(__fsub_rn(__fmul_rn(-r.dx, c.z), __fmul_rn(c.x, -r.dz)), k);
-	const float i21 = __fmul_rn(-__fsub_rn(__fmul_rn(-r.dx, c.y), __fmul_rn(c.x, -r.dy)), k);
-	u = __fadd_rn(__fadd_rn(__fmul_rn(i01, spx), __fmul_rn(i11, spy)), __fmul_rn(i21, spz));
-	if (!(u >= 0.0f))
+	// Rows 1 and 2 of the inverse give u and v.
+	const unsigned long long kk = pair2(k, k);
+	unpair2(mul2(X, dz), p0, p1);
+	unpair2(mul2(dx, Z), q0, q1);
+	const float P = __fsub_rn(p0, q0), Q = __fsub_rn(p1, q1);
+	unpair2(mul2(X, dy), p0, p1);
+	unpair2(mul2(dx, Y), q0, q1);
+	const float S = __fsub_rn(p0, q0), T = __fsub_rn(p1, q1);
+	float u0, u1, u2, v0, v1, v2;
+	unpair2(mul2(mul2(pair2(A, B), kk), pair2(spx, spx)), u0, v0);
+	unpair2(mul2(mul2(pair2(P, Q), kk), pair2(spy, spy)), u1, v1);
+	unpair2(mul2(mul2(pair2(S, T), kk), pair2(spz, spz)), u2, v2);
+	u = __fsub_rn(__fsub_rn(u1, u0), u2);
+	v = __fadd_rn(__fsub_rn(v0, v1), v2);
+	if (!kStraight && !((u >= 0.0f) & (v >= 0.0f) & (__fadd_rn(u, v) <= 1.0f)))
 		return false;
-	const float i02 = __fmul_rn(B, k);
-	const float i12 = __fmul_rn(-__fsub_rn(__fmul_rn(-r.dx, b.z), __fmul_rn(b.x, -r.dz)), k);
-	const float i22 = __fmul_rn(__fsub_rn(__fmul_rn(-r.dx, b.y), __fmul_rn(b.x, -r.dy)), k);
-	v = __fadd_rn(__fadd_rn(__fmul_rn(i02, spx), __fmul_rn(i12, spy)), __fmul_rn(i22, spz));
-	if (!(v >= 0.0f) || !(__fadd_rn(u, v) <= 1.0f))
-		return false;
-	const float i00 = __fmul_rn(c00, k);
-	const float i10 = __fmul_rn(-__fsub_rn(__fmul_rn(b.x, c.z), __fmul_rn(c.x, b.z)), k);
-	const float i20 = __fmul_rn(__fsub_rn(__fmul_rn(b.x, c.y), __fmul_rn(c.x, b.y)), k);
+	const float i00 = __fmul_rn(c.z, k);
+	const float i10 = __fmul_rn(-__fsub_rn(__fmul_rn(b.y, c.x), __fmul_rn(b.x, c.y)), k);
+	const float i20 = __fmul_rn(__fsub_rn(__fmul_rn(b.y, b.z), __fmul_rn(b.x, b.w)), k);
 	t = __fadd_rn(__fadd_rn(__fmul_rn(i00, spx), __fmul_rn(i10, spy)), __fmul_rn(i20, spz));
-	return t > 1e-5f;
+	if (!kStraight)
+		return t > 1e-5f;
+	return !(fabsf(det) < 1e-8f) & (u >= 0.0f) & (v >= 0.0f) & (__fadd_rn(u, v) <= 1.0f) & (t > 1e-5f);
 }
 
 __device__ __forceinline__ int leaf_start(int ref) { return (~ref) >> 3; }
@@ -174,7 +219,7 @@ __device__ __forceinline__ bool bad_leaf(const SceneView &s, int start, int coun
 // Closest hit. `ignore` is an original triangle index to skip (-1 = none).
 // `err` is set to 1 if the stack bound would be exceeded (the host rejects
 // trees deeper than the bound, so this only reports corrupted input).
-template <int kOrder>
+template <int kOrder, bool kStraight = false>
 __device__ __forceinline__ HitRec trace_closest(const SceneView &s, const RayPre &r, int ignore, int &err) {
 	HitRec h;
 	h.idx = -1;
@@ -283,7 +328,7 @@ __device__ __forceinline__ HitRec trace_closest(const SceneView &s, const RayPre
 			const float4 b = __ldg(tp + 1);
 			const float4 c = __ldg(tp + 2);
 			float t, u, v;
-			if (!tri_test(a, b, c, r, t, u, v))
+			if (!tri_test<false, kStraight>(a, b, c, r, t, u, v))
 				continue;
 			if (kOrder == kOrderReference) {
 				if (t < h.t) {
@@ -291,10 +336,10 @@ __device__ __forceinline__ HitRec trace_closest(const SceneView &s, const RayPre
 					h.t = t;
 					h.u = u;
 					h.v = v;
-					h.rank = __float_as_int(b.w);
+					h.rank = __float_as_int(c.w);
 				}
 			} else {
-				const int rk = __float_as_int(b.w);
+				const int rk = __float_as_int(c.w);
 				if (t < h.t || (t == h.t && rk < h.rank)) {
 					h.idx = ti;
 					h.t = t;
@@ -386,30 +431,6 @@ __device__ __forceinline__ bool trace_any(const SceneView &s, const RayPre &r, f
 // zero or subnormal direction component, where a slab product can be NaN) take the 2-wide
 // path instead.
 
-// Paired single-precision arithmetic of sm_100 (PTX sub/mul .rn.f32x2): two independently,
-// correctly rounded IEEE operations per instruction, so the slab products keep the
-// reference's bits at half the instruction count. A product may only feed scalar sums: ptxas
-// contracts mul.rn.f32x2 into a following packed sum in spite of .rn (measured), while the
-// slab's order, differences first, leaves it nothing to contract.
-__device__ __forceinline__ unsigned long long pair2(float lo, float hi) {
-	unsigned long long r;
-	asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-	return r;
-}
-__device__ __forceinline__ void unpair2(unsigned long long v, float &lo, float &hi) {
-	asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b) {
-	unsigned long long r;
-	asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-	return r;
-}
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
-	unsigned long long r;
-	asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-	return r;
-}
-
 // Three-input min / max of sm_100 (PTX min.f32 / max.f32 with three sources).
 __device__ __forceinline__ float max3(float a, float b, float c) {
 	float r;
@@ -421,7 +442,6 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
 	asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
 	return r;
 }
-
 
 // The ray's origin and inverse direction duplicated into pairs, and per axis the byte
 // offset in a 4-wide node of the row that holds the planes the ray meets first (lo for a
@@ -626,17 +646,15 @@ __device__ __forceinline__ HitRec trace_closest4_spec(const SceneView &s, const 
 					const float4 *tp = s.tris + 3 * static_cast<size_t>(p);
 					const float4 a = __ldg(tp + 0);
 					const int ti = __float_as_int(a.w);
-					if (ti == ignore)
-						continue;
 					const float4 b = __ldg(tp + 1);
 					const float4 c = __ldg(tp + 2);
 					float t, u, v;
-					if (tri_test<true>(a, b, c, r, t, u, v) && t < h.t) {
+					if (tri_test<true>(a, b, c, r, t, u, v) && t < h.t && ti != ignore) {
 						h.idx = ti;
 						h.t = t;
 						h.u = u;
 						h.v = v;
-						h.rank = __float_as_int(b.w);
+						h.rank = __float_as_int(c.w);
 					}
 				}
 			}
@@ -843,12 +861,10 @@ __device__ __forceinline__ bool trace_any4_spec(const SceneView &s, const RayPre
 			for (int p = start; p < start + count; p++) {
 				const float4 *tp = s.tris + 3 * static_cast<size_t>(p);
 				const float4 a = __ldg(tp + 0);
-				if (__float_as_int(a.w) == ignore)
-					continue;
 				const float4 b = __ldg(tp + 1);
 				const float4 c = __ldg(tp + 2);
 				float t, u, v;
-				if (tri_test<true>(a, b, c, r, t, u, v) && t < tmax)
+				if (tri_test<true>(a, b, c, r, t, u, v) && t < tmax && __float_as_int(a.w) != ignore)
 					return true;
 			}
 			leaf = kNoRef;
@@ -869,7 +885,7 @@ __device__ __forceinline__ bool trace_any4_spec(const SceneView &s, const RayPre
 // gathered, as in the functions above) and, once kStreamRefill lanes are idle, gives each of
 // them the next ray; a round's descent ends when fewer than kStreamActive lanes are left in
 // it (while there are rays to refill from). The order of a ray's own steps is unchanged.
-// 2M unordered closest hits: 1.09 -> 0.88 ms (12.3 lanes); without the second rule 0.98, and
+// 2M unordered closest hits: 1.09 -> 0.88 ms (12.3 lanes; 0.78 with tri_test's straight form); without the second rule 0.98, and
 // 0.90 to 0.93 with other numbers of lanes (8 and 12, 8 and 20, 12 and 24). Where neighbours
 // already take the same way the exchange costs more than it gives: any hits towards one
 // light 0.49 -> 0.48 ms, the wavefront's binned rays 24.7 -> 33 ms a frame, a scene of 36
@@ -941,7 +957,7 @@ __device__ __forceinline__ void trace_closest_stream(const SceneView &s, Stack &
 				cur = leaf = kNoRef;
 				float te;
 				if (!bounded_ray(s, r)) {
-					sink(trace_closest<kOrderReference>(s, r, ignore, err));
+					sink(trace_closest<kOrderReference, true>(s, r, ignore, err));
 				} else if (slab(s.root_lo[0], s.root_hi[0], s.root_lo[1], s.root_hi[1], s.root_lo[2], s.root_hi[2], r,
 				                te)) {
 					r2 = make_pair_ray(r);
@@ -1011,17 +1027,15 @@ __device__ __forceinline__ void trace_closest_stream(const SceneView &s, Stack &
 					const float4 *tp = s.tris + 3 * static_cast<size_t>(p);
 					const float4 a = __ldg(tp + 0);
 					const int ti = __float_as_int(a.w);
-					if (ti == ignore)
-						continue;
 					const float4 b = __ldg(tp + 1);
 					const float4 c = __ldg(tp + 2);
 					float t, u, v;
-					if (tri_test<true>(a, b, c, r, t, u, v) && t < h.t) {
+					if (tri_test<true, true>(a, b, c, r, t, u, v) && t < h.t && ti != ignore) {
 						h.idx = ti;
 						h.t = t;
 						h.u = u;
 						h.v = v;
-						h.rank = __float_as_int(b.w);
+						h.rank = __float_as_int(c.w);
 					}
 				}
 			}
@@ -1150,7 +1164,7 @@ __device__ __forceinline__ bool trav_step(TravState &ts, const SceneView &s, int
 			ts.h.t = t;
 			ts.h.u = u;
 			ts.h.v = v;
-			ts.h.rank = __float_as_int(bb.w);
+			ts.h.rank = __float_as_int(c.w);
 		}
 	}
 	return true;
@@ -1250,7 +1264,7 @@ __device__ bool count_reference_query(const SceneView &s, const RayPre &r, int i
 					h.t = t;
 					h.u = u;
 					h.v = v;
-					h.rank = __float_as_int(b.w);
+					h.rank = __float_as_int(c.w);
 				}
 			}
 			continue;
