@@ -829,12 +829,18 @@ __device__ __forceinline__ void deposit(float *image, int pix, V3 v) {
 	atomicAdd(image + 3 * static_cast<size_t>(pix) + 2, v.z);
 }
 
-// One Markov chain per thread (src/Metropolis.cpp:127-173 per chain).
-__global__ void __launch_bounds__(128) k_mlt_chains(SceneView sv, const float4 *__restrict__ ref_shade, GiParams p,
+// One Markov chain per thread (src/Metropolis.cpp:127-173 per chain); with `spread`, per 2^spread
+// threads, so that few chains reach more of the chip's schedulers and share their warps with
+// fewer paths of other lengths. A step waits on one path's dependent loads and tests. With
+// more chains than fit at once, nine blocks an SM (56 registers and some spills) hide more of
+// that than the registers do; with fewer the registers do.
+template <int kBlocks>
+__global__ void __launch_bounds__(128, kBlocks) k_mlt_chains(SceneView sv, const float4 *__restrict__ ref_shade, GiParams p,
                                                     const double *__restrict__ cdf, const double *__restrict__ total,
-                                                    const uint8_t *__restrict__ len, float *image, int *status) {
-	const int ch = blockIdx.x * blockDim.x + threadIdx.x;
-	if (ch >= p.chains)
+                                                    const uint8_t *__restrict__ len, float *image, int spread, int *status) {
+	const unsigned thread = blockIdx.x * blockDim.x + threadIdx.x;
+	const int ch = static_cast<int>(thread >> spread);
+	if ((thread & ((1u << spread) - 1u)) || ch >= p.chains)
 		return;
 	const double tot = *total;
 	if (!(tot > 0.0))
@@ -872,10 +878,11 @@ __global__ void __launch_bounds__(128) k_mlt_chains(SceneView sv, const float4 *
 		const bool large = W(0) < p_large;
 		int pn = cn;
 		for (int m = 0; m < cn; m++) {
+			const float a0 = W(2 + 2 * m); // drawn once for the lanes of both kinds
 			if (large) {
-				prop[m] = W(2 + 2 * m);
+				prop[m] = a0;
 			} else {
-				const float a0 = W(2 + 2 * m), a1 = W(3 + 2 * m);
+				const float a1 = W(3 + 2 * m);
 				float v = cur[m] + sigma * gi_normal(a0, a1);
 				v = v - floorf(v);
 				prop[m] = v;
@@ -1043,6 +1050,13 @@ size_t mlt_scratch_bytes(const GiParams &p) {
 	       align256(static_cast<size_t>(p.width) * p.height * 3 * 4);
 }
 
+// Up to two blocks' worth of chains an SM take the kernel without a register cap, spread over
+// as many threads; more the capped one. On the room: 4M mutations (250 000 chains) 7.6 ms without
+// the cap, 6.9 with it, 1M (62 500) 3.2 and 2.3, 500 000 (31 250) 1.6 and 1.85; 20 000
+// (1 250 chains) 1.41 ms unspread, 1.21 / 1.03 / 0.91 / 0.92 over 4 / 8 / 16 / 32 threads a
+// chain; 31 250 over two threads 2.9.
+constexpr int kMltRoom = 148 * 2 * 128, kMltSpread = 4;
+
 cudaError_t launch_mlt(const SceneView &sv, const float4 *ref_shade, const GiParams &p, void *scratch, uint32_t *argb,
                        float *rgb, double *b_out, int *status, cudaStream_t st) {
 	const size_t b = static_cast<size_t>(p.bootstrap);
@@ -1066,8 +1080,15 @@ cudaError_t launch_mlt(const SceneView &sv, const float4 *ref_shade, const GiPar
 		k_mlt_cdf<<<1, 1024, 0, st>>>(lum, p.bootstrap, cdf, total);
 	}
 	TraceRange r("chains");
-	k_mlt_chains<<<static_cast<unsigned>((p.chains + 127) / 128), 128, 0, st>>>(sv, ref_shade, p, cdf, total, len,
-	                                                                          image, status);
+	const bool many = p.chains > kMltRoom;
+	int spread = 0;
+	while (spread < kMltSpread && (static_cast<long>(p.chains) << (spread + 1)) <= kMltRoom)
+		spread++;
+	const unsigned grid = static_cast<unsigned>(((static_cast<long>(p.chains) << spread) + 127) / 128);
+	if (many)
+		k_mlt_chains<9><<<grid, 128, 0, st>>>(sv, ref_shade, p, cdf, total, len, image, spread, status);
+	else
+		k_mlt_chains<1><<<grid, 128, 0, st>>>(sv, ref_shade, p, cdf, total, len, image, spread, status);
 	const long g = std::min<long>((npix + 255) / 256, 148 * 16);
 	k_mlt_resolve<<<static_cast<unsigned>(g), 256, 0, st>>>(p, image, total, argb, rgb, b_out);
 	return cudaGetLastError();
