@@ -283,8 +283,10 @@ __device__ void record_path(Ctx &c, V3 origin, V3 direction, Rng &rng, const Def
 }
 
 // Persistent: a lane that has finished its pixel takes the next one, so lanes
-// whose paths end early do not idle until the warp's longest pixel is done.
-__global__ void __launch_bounds__(128) k_ref_paths(SceneView sv, const float4 *__restrict__ ref_shade,
+// whose paths end early do not idle until the warp's longest pixel is done. Eight blocks an
+// SM: 1280 x 720 x 8 samples over 328 000 triangles 10.1 -> 9.7 ms, 1080p x 2 over 1.31M
+// 4.1 -> 3.9 (seven and nine 4.04 and 4.01).
+__global__ void __launch_bounds__(128, 8) k_ref_paths(SceneView sv, const float4 *__restrict__ ref_shade,
                                                    const RefParams *__restrict__ params, DeferView dv, int *status) {
 	const RefParams &p = *params;
 	Ctx c{sv, ref_shade, &p, 0};
@@ -315,13 +317,20 @@ __global__ void k_shade_count(DeferView dv) {
 	     e += static_cast<long>(gridDim.x) * blockDim.x)
 		atomicAdd(dv.bins + dv.key[e], 1u);
 }
+// Each thread's 32 bins are read at once, not one after another: 53 -> 8 us.
 __global__ void __launch_bounds__(1024) k_shade_scan(DeferView dv) {
 	constexpr int kBins = 1 << kShadeKeyBits, kPer = kBins / 1024;
 	__shared__ unsigned part[1024];
+	static_assert(kPer % 4 == 0, "the bins move four at a time");
 	const int t = threadIdx.x;
+	uint4 *own = reinterpret_cast<uint4 *>(dv.bins) + t * (kPer / 4); // dv.bins starts a 256-byte block
+	uint4 c[kPer / 4];
 	unsigned sum = 0;
-	for (int j = 0; j < kPer; j++)
-		sum += dv.bins[t * kPer + j];
+#pragma unroll
+	for (int j = 0; j < kPer / 4; j++) {
+		c[j] = own[j];
+		sum += c[j].x + c[j].y + c[j].z + c[j].w;
+	}
 	part[t] = sum;
 	__syncthreads();
 	for (int off = 1; off < 1024; off <<= 1) {
@@ -331,10 +340,11 @@ __global__ void __launch_bounds__(1024) k_shade_scan(DeferView dv) {
 		__syncthreads();
 	}
 	unsigned run = part[t] - sum; // exclusive prefix of this thread's bins
-	for (int j = 0; j < kPer; j++) {
-		const unsigned c = dv.bins[t * kPer + j];
-		dv.bins[t * kPer + j] = run;
-		run += c;
+#pragma unroll
+	for (int j = 0; j < kPer / 4; j++) {
+		const uint4 v = c[j];
+		own[j] = make_uint4(run, run + v.x, run + v.x + v.y, run + v.x + v.y + v.z);
+		run += v.x + v.y + v.z + v.w;
 	}
 }
 __global__ void k_shade_scatter(DeferView dv) {
@@ -349,7 +359,8 @@ __global__ void k_shade_scatter(DeferView dv) {
 }
 
 // Eight blocks an SM: the 1.31M-triangle 1080p x 2 spp frame's shadow pass takes 12.2 ms,
-// against 12.7 at the 72 registers (seven blocks) it takes uncapped.
+// against 12.7 at the 72 registers (seven blocks) it takes uncapped (since then 5.0 against
+// 5.4; six, seven, nine and ten blocks 5.66, 5.59, 5.22 and 5.23).
 __global__ void __launch_bounds__(128, 8) k_ref_shadow(SceneView sv, const RefParams *__restrict__ params, DeferView dv,
                                                     int *status) {
 	const RefParams &p = *params;
