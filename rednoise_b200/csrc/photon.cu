@@ -359,45 +359,112 @@ __device__ V3 gather(const PhotonMapView &m, V3 point, V3 normal) {
 	return irradiance(m, sum);
 }
 
-// One gather by a whole warp: 32 photons are loaded and tested at a time, the next 32 on
-// their way, and the accepted ones' powers are added in order from the lanes that hold
-// them (every lane forms the same sum).
-__device__ V3 gather_warp(const PhotonMapView &m, V3 point, V3 normal) {
-	const int lane = threadIdx.x & 31;
+// One gather by a whole block of 128 threads, every one of which passes the same point and
+// normal; thread 0 returns the result. Three warps load and test 128 photons each and leave
+// the accepted ones' powers, in order, in their part of a batch; meanwhile the first three
+// lanes of the other warp add up the batch before, one channel each.
+constexpr int kBatchPart = 128;
+struct GatherBatch {
+	float power[2][3][3][kBatchPart]; // batch parity, warp, channel
+	int count[2][3];
+};
+__device__ V3 gather_block(const PhotonMapView &m, V3 point, V3 normal, GatherBatch &batch) {
+	const int lane = threadIdx.x & 31, part = static_cast<int>(threadIdx.x >> 5) - 1; // -1: the adding warp
 	const float r2 = m.radius * m.radius;
 	const CellBlock b = cell_block(m, point);
 	uint32_t my_lo = 0, my_hi = 0;
 	if (lane < b.runs())
 		cell_run(m, b, lane, my_lo, my_hi);
-	V3 sum = mk(0.0f, 0.0f, 0.0f);
+	float sum = 0.0f;
+	int parity = 0;
 	for (int run = 0; run < b.runs(); run++) {
 		const uint32_t lo = __shfl_sync(0xffffffffu, my_lo, run), hi = __shfl_sync(0xffffffffu, my_hi, run);
-		if (lo >= hi)
-			continue;
-		uint32_t e = min(lo + lane, hi - 1);
-		float4 pp = __ldg(m.pos + e), pd = __ldg(m.dir + e), pw = __ldg(m.pw + e);
-		for (uint32_t at = lo; at < hi; at += 32) {
-			e = min(at + 32 + lane, hi - 1);
-			const float4 np = __ldg(m.pos + e), nd = __ldg(m.dir + e), nw = __ldg(m.pw + e);
-			unsigned in = __ballot_sync(0xffffffffu, at + lane < hi && accepts(pp, pd, point, normal, r2));
-			while (in) {
-				const int j = __ffs(in) - 1;
-				in &= in - 1;
-				add_power(sum, __shfl_sync(0xffffffffu, pw.x, j), __shfl_sync(0xffffffffu, pw.y, j),
-				          __shfl_sync(0xffffffffu, pw.z, j));
+		for (uint32_t at = lo; at < hi; at += 3 * kBatchPart, parity ^= 1) {
+			if (part >= 0) {
+				int n = 0;
+#pragma unroll
+				for (int k = 0; k < kBatchPart / 32; k++) {
+					const uint32_t e = at + part * kBatchPart + k * 32 + lane, in_range = min(e, hi - 1);
+					const float4 pp = __ldg(m.pos + in_range), pd = __ldg(m.dir + in_range), pw = __ldg(m.pw + in_range);
+					const bool ok = e < hi && accepts(pp, pd, point, normal, r2);
+					const unsigned in = __ballot_sync(0xffffffffu, ok);
+					if (ok) {
+						const int to = n + __popc(in & ((1u << lane) - 1u));
+						batch.power[parity][part][0][to] = pw.x;
+						batch.power[parity][part][1][to] = pw.y;
+						batch.power[parity][part][2][to] = pw.z;
+					}
+					n += __popc(in);
+				}
+				if (lane == 0)
+					batch.count[parity][part] = n;
 			}
-			pp = np;
-			pd = nd;
-			pw = nw;
+			// the batch is complete, and the adding warp is done with the one before
+			__syncthreads();
+			if (part < 0 && lane < 3) {
+				for (int w = 0; w < 3; w++) {
+					const float *q = batch.power[parity][w][lane];
+					const int n = batch.count[parity][w];
+					int k = 0;
+					for (; k + 8 <= n; k += 8) {
+						const float4 u = *reinterpret_cast<const float4 *>(q + k), v = *reinterpret_cast<const float4 *>(q + k + 4);
+						sum = sum + u.x;
+						sum = sum + u.y;
+						sum = sum + u.z;
+						sum = sum + u.w;
+						sum = sum + v.x;
+						sum = sum + v.y;
+						sum = sum + v.z;
+						sum = sum + v.w;
+					}
+					for (; k < n; k++)
+						sum = sum + q[k];
+				}
+			}
 		}
 	}
-	return irradiance(m, sum);
+	const V3 all = mk(__shfl_sync(0xffffffffu, sum, 0), __shfl_sync(0xffffffffu, sum, 1),
+	                  __shfl_sync(0xffffffffu, sum, 2));
+	return irradiance(m, all);
 }
 
-// A warp's gathers, one per lane, where most lanes stand in the same cell: the lanes of
-// one cell share its photons, which the warp copies 32 at a time to its tile in shared
-// memory (the next 32 on their way to registers) and every lane then walks for its own
-// point. Other cells' lanes take their turns.
+// The box of the points of the lanes in `mine`, and what is farther from it than the gather's
+// radius. far() is exact in the sense that matters: what it calls far, accepts() rejects for
+// every point in the box. Its margin covers the rounding of both sums of squares (a few
+// 2^-24; the radius is kept away from the subnormals), and what is not finite is never far,
+// since accepts() takes a distance that is not a number.
+struct PointBox {
+	float lo[3], hi[3], limit;
+	static __device__ __forceinline__ int ordered(float x) {
+		const int b = __float_as_int(x);
+		return b ^ ((b >> 31) & 0x7fffffff);
+	}
+	static __device__ __forceinline__ float unordered(int b) { return __int_as_float(b ^ ((b >> 31) & 0x7fffffff)); }
+	__device__ __forceinline__ PointBox(V3 p, bool mine, float r2) {
+		const float inf = __int_as_float(0x7f800000), q[3] = {p.x, p.y, p.z};
+		const bool finite = fabsf(p.x) < inf && fabsf(p.y) < inf && fabsf(p.z) < inf;
+		for (int a = 0; a < 3; a++) {
+			lo[a] = unordered(__reduce_min_sync(0xffffffffu, ordered(mine ? q[a] : inf)));
+			hi[a] = unordered(__reduce_max_sync(0xffffffffu, ordered(mine ? q[a] : -inf)));
+		}
+		limit = __any_sync(0xffffffffu, mine && !finite) || !(r2 > 1e-30f) ? inf : r2 * 1.00001f;
+	}
+	__device__ __forceinline__ bool far(const float4 &p) const {
+		const float x = fmaxf(fmaxf(lo[0] - p.x, p.x - hi[0]), 0.0f), y = fmaxf(fmaxf(lo[1] - p.y, p.y - hi[1]), 0.0f),
+		            z = fmaxf(fmaxf(lo[2] - p.z, p.z - hi[2]), 0.0f);
+		const float sum = p.x + p.y + p.z;
+		return x * x + y * y + z * z > limit && sum - sum == 0.0f;
+	}
+};
+
+// A warp's gathers, one per lane, where most lanes stand close together in the same cell: the
+// lanes of one cell share its photons, which the warp reads 32 at a time (the next 32 on their
+// way to registers). Those that are too far from every lane's point stay out, the others
+// go in order to the warp's tile in shared memory, which every lane then walks for its own
+// point. Other cells' lanes take their turns. A sphere of the radius in 27 cells: of
+// the photons a lone point tests about two thirds are too far; leaving those of them out that no
+// point of the warp needs took the kernel (before the blocks below) from 8.2 to 6.8 ms at
+// 200 000 photons.
 __device__ V3 gather_lanes(const PhotonMapView &m, V3 point, V3 normal, bool live, float4 (*tile)[32]) {
 	const int lane = threadIdx.x & 31;
 	const float r2 = m.radius * m.radius;
@@ -410,6 +477,7 @@ __device__ V3 gather_lanes(const PhotonMapView &m, V3 point, V3 normal, bool liv
 		                               __shfl_sync(0xffffffffu, own.z, lead));
 		const bool mine = live && own.x == b.x && own.y == b.y && own.z == b.z;
 		todo &= ~__ballot_sync(0xffffffffu, mine);
+		const PointBox box(point, mine, r2);
 		uint32_t my_lo = 0, my_hi = 0;
 		if (lane < b.runs())
 			cell_run(m, b, lane, my_lo, my_hi);
@@ -420,16 +488,20 @@ __device__ V3 gather_lanes(const PhotonMapView &m, V3 point, V3 normal, bool liv
 			uint32_t e = min(lo + lane, hi - 1);
 			float4 pp = __ldg(m.pos + e), pd = __ldg(m.dir + e), pw = __ldg(m.pw + e);
 			for (uint32_t at = lo; at < hi; at += 32) {
-				__syncwarp();
-				tile[0][lane] = pp;
-				tile[1][lane] = pd;
-				tile[2][lane] = pw;
+				const bool near = at + lane < hi && !box.far(pp);
+				const unsigned in = __ballot_sync(0xffffffffu, near);
+				if (near) {
+					const int to = __popc(in & ((1u << lane) - 1u));
+					tile[0][to] = pp;
+					tile[1][to] = pd;
+					tile[2][to] = pw;
+				}
 				__syncwarp();
 				e = min(at + 32 + lane, hi - 1);
 				pp = __ldg(m.pos + e);
 				pd = __ldg(m.dir + e);
 				pw = __ldg(m.pw + e);
-				const int cnt = static_cast<int>(min(hi - at, 32u));
+				const int cnt = __popc(in);
 				if (mine) {
 #pragma unroll 4
 					for (int k = 0; k < cnt; k++) {
@@ -438,6 +510,7 @@ __device__ V3 gather_lanes(const PhotonMapView &m, V3 point, V3 normal, bool liv
 							add_power(sum, w.x, w.y, w.z);
 					}
 				}
+				__syncwarp();
 			}
 		}
 	}
@@ -668,8 +741,18 @@ __global__ void __launch_bounds__(128) k_photon_hits(SceneView sv, const float4 
 
 // Direct light and the gather's sort key of n requests, kGroup lanes to a request (1, or 10:
 // a disk or rectangle light's nine visibility rays run side by side). The key orders the
-// requests by the photons they test, most first (the upper 16 bits of that number as a
-// float), and within that by a hash of their cell.
+// requests by the photons they test, most first (12 bits: exponent and 7 bits of mantissa of
+// that number), within that by a hash of their cell, and within a cell by place.
+__device__ __forceinline__ uint32_t sub_cell(float x, float y, float z) {
+	const float q[3] = {x, y, z}; // 12-bit Morton code of a place in the unit cell
+	uint32_t code = 0;
+	for (int a = 0; a < 3; a++) {
+		const uint32_t c = static_cast<uint32_t>(fminf(fmaxf(q[a] * 16.0f, 0.0f), 15.0f));
+		for (int b = 0; b < 4; b++)
+			code |= ((c >> b) & 1u) << (3 * b + a);
+	}
+	return code;
+}
 constexpr int kDirectLanes = 10;
 template <int kGroup>
 __global__ void __launch_bounds__(128) k_photon_direct(SceneView sv, const float4 *__restrict__ ref_shade,
@@ -747,28 +830,33 @@ __global__ void __launch_bounds__(128) k_photon_direct(SceneView sv, const float
 			cell_run(m, b, lane, lo, hi);
 		const uint32_t tests = __reduce_add_sync(0xffffffffu, hi - lo);
 		if (mine && g == 0) {
-			const uint32_t size = static_cast<uint32_t>(__float_as_int(static_cast<float>(tests))) >> 16;
+			// 1.0f >> 16 = 0x3F80: a size of 0 stays 0, 1 becomes 1, 2^31 3969
+			const uint32_t bits = static_cast<uint32_t>(__float_as_int(static_cast<float>(tests))) >> 16;
+			const uint32_t size = bits < 0x3F80u ? 0u : min(bits - 0x3F7Fu, 0xFFFu);
 			const uint32_t hash = static_cast<uint32_t>(b.x) * 73856093u ^ static_cast<uint32_t>(b.y) * 19349663u ^
 			                      static_cast<uint32_t>(b.z) * 83492791u;
-			q.key[r] = ((0xFFFFu - size) << 16) | (hash >> 16);
+			q.key[r] = ((0xFFFu - size) << 20) | ((hash >> 24) << 12) |
+			           sub_cell(point.x / m.cell - static_cast<float>(b.x), point.y / m.cell - static_cast<float>(b.y),
+			                    point.z / m.cell - static_cast<float>(b.z));
 		}
 	}
 }
 
-// The first kWarpGathers requests (the largest) get a warp each, the others a lane each of
-// warps that share a cell's photons (gather_lanes). A lane adds its photons one by one, so
-// the request that tests the most (under the light: nearly all photons there are) bounds the
-// kernel: by a thread of its own it took 35 ms of 200 000 photons' 1280 x 720 frame, by a
-// warp 1; but a warp per request costs four times the instructions, so only as many as fill
-// the chip once get one: with 148 * 8, 16, 32 and 64 the kernel takes 14.1, 13.3, 8.5 and
-// 8.6 ms.
-constexpr uint32_t kWarpGathers = 148 * 32;
+// The first kBlockGathers requests (the largest) get a block each, the others a lane each of
+// warps that share a cell's photons (gather_lanes). A request's photons are added one by
+// one, so those that test the most (under the light: nearly all photons there are) bound the
+// kernel: by threads of their own they took 35 ms of 200 000 photons' 1280 x 720 frame, by
+// warps 6.8 (at the best number of them, 148 * 32), by blocks 10.2, 6.7, 5.6 and 6.0 for the
+// first 148 * 16, 32, 64 and 128. Warps of fewer lanes for the requests after those: 6.0 and up.
+constexpr uint32_t kBlockGathers = 148 * 64;
 __global__ void __launch_bounds__(128) k_photon_gather(PhotonMapView m, PhotonRequests q, uint32_t n) {
-	__shared__ float4 tile[4][3][32];
+	__shared__ union {
+		float4 tile[4][3][32];
+		GatherBatch batch;
+	} sh;
 	const int warp = threadIdx.x >> 5;
-	const bool whole = blockIdx.x < kWarpGathers / 4;
-	const uint32_t i = whole ? blockIdx.x * 4 + warp
-	                         : kWarpGathers + (blockIdx.x - kWarpGathers / 4) * blockDim.x + threadIdx.x;
+	const bool whole = blockIdx.x < kBlockGathers;
+	const uint32_t i = whole ? blockIdx.x : kBlockGathers + (blockIdx.x - kBlockGathers) * blockDim.x + threadIdx.x;
 	const bool live = i < n;
 	if (whole && !live)
 		return;
@@ -780,8 +868,10 @@ __global__ void __launch_bounds__(128) k_photon_gather(PhotonMapView m, PhotonRe
 		point = mk(pt.x, pt.y, pt.z);
 		normal = mk(nn.x, nn.y, nn.z);
 	}
-	const V3 g = whole ? gather_warp(m, point, normal) : gather_lanes(m, point, normal, live, tile[warp]);
-	if (!live || (whole && (threadIdx.x & 31) != 0))
+	if (whole)
+		__syncthreads(); // thread 0 writes q.point[r] at its end: every thread has read it
+	const V3 g = whole ? gather_block(m, point, normal, sh.batch) : gather_lanes(m, point, normal, live, sh.tile[warp]);
+	if (!live || (whole && threadIdx.x != 0))
 		return;
 	const float4 al = q.albedo[r], d = q.direct[r];
 	const V3 v = mk(d.x, d.y, d.z) + mk(al.x, al.y, al.z) * g;
@@ -1027,9 +1117,8 @@ cudaError_t launch_photon_mapped(const SceneView &sv, const float4 *ref_shade, c
 			                                    static_cast<int>(n), 0, 32, st);
 			if (e != cudaSuccess)
 				return e;
-			const unsigned lanes = n > kWarpGathers ? n - kWarpGathers : 0;
-			k_photon_gather<<<kWarpGathers / 4 + static_cast<unsigned>(ceil_div(static_cast<long>(lanes), bs)), bs, 0, st>>>(
-			    m, q, n);
+			const unsigned whole = std::min<unsigned>(n, kBlockGathers), lanes = n - whole;
+			k_photon_gather<<<whole + static_cast<unsigned>(ceil_div(static_cast<long>(lanes), bs)), bs, 0, st>>>(m, q, n);
 		}
 		k_photon_hits<false><<<blocks, 128, 0, st>>>(sv, ref_shade, d_params, q, y0, y1, argb, status);
 		y0 = y1;

@@ -1,5 +1,5 @@
-"""Writes photon_canvases.npz: the photon mapper's canvases of tests/photon_scenes.py (needs the
-GPU). Kept from the build whose photon mapper was checked against the reference's own."""
+"""Writes photon_canvases.npz, the photon mapper's canvases of tests/photon_scenes.py (needs the GPU);
+photon_lanes.npz holds those of tests/test_photon_lanes_gpu.py from the same build. Kept from the build whose photon mapper was checked against the reference's own."""
 import os
 import sys
 
