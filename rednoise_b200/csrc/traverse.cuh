@@ -885,11 +885,11 @@ __device__ __forceinline__ bool trace_any4_spec(const SceneView &s, const RayPre
 // gathered, as in the functions above) and, once kStreamRefill lanes are idle, gives each of
 // them the next ray; a round's descent ends when fewer than kStreamActive lanes are left in
 // it (while there are rays to refill from). The order of a ray's own steps is unchanged.
-// 2M unordered closest hits: 1.09 -> 0.88 ms (12.3 lanes; 0.78 with tri_test's straight form); without the second rule 0.98, and
-// 0.90 to 0.93 with other numbers of lanes (8 and 12, 8 and 20, 12 and 24). Where neighbours
-// already take the same way the exchange costs more than it gives: any hits towards one
-// light 0.49 -> 0.48 ms, the wavefront's binned rays 24.7 -> 33 ms a frame, a scene of 36
-// triangles 0.34 -> 0.41 ms.
+// 2M unordered closest hits: 1.09 -> 0.88 ms (12.3 lanes), 0.78 with tri_test's straight form;
+// without the second rule 0.98, and 0.90 to 0.93 with other numbers of lanes (8 and 12, 8 and
+// 20, 12 and 24). Where neighbours already take the same way the exchange costs more than it
+// gives: any hits towards one light 0.49 -> 0.48 ms, the wavefront's binned rays 24.7 -> 33 ms
+// a frame, a scene of 36 triangles 0.34 -> 0.41 ms.
 // source(want, idle, ...) gives every lane with want set its next ray, false if there is none
 // (it is called by all lanes; idle is the mask of those that want one); sink takes a finished
 // ray's result. Every lane of the warp must call this function; rays that are not

@@ -72,9 +72,9 @@ constexpr int kWfShortStack = 8;
 constexpr size_t kWfExtendSmem = static_cast<size_t>(kWfShortStack) * 128 * sizeof(unsigned long long);
 constexpr size_t kWfShadowSmem = static_cast<size_t>(kWfShortStack) * 128 * sizeof(int);
 
-// No register cap: at 64 registers (eight blocks an SM) the closest-hit stage of the
-// 1.31M-triangle 1080p x 32 spp frame takes 47.9 ms; capped at 56 (nine blocks) 50.6,
-// at 72 (seven) 49.4.
+// No register cap: the closest-hit stage of the 1.31M-triangle 1080p x 32 spp frame takes 22.9
+// ms at the 56 registers it comes to; asked for six, seven, eight, nine and ten blocks an SM
+// the compiler schedules it otherwise and it takes 26.5, 24.8, 24.4, 23.4 and 24.3.
 template <int kOrder>
 __global__ void __launch_bounds__(128) k_wf_extend(const WfJob *__restrict__ jobs, WfPool pool, int k,
                                                    const int *__restrict__ q, int only_job, int *status) {
