@@ -79,7 +79,7 @@ rn_status prepare_scene(rn_scene *s) {
 	// The 4-wide tree, while this thread lays out the reference's and the shading records. A
 	// scene of few triangles keeps the reference's shape: there is little to skip above its
 	// leaves, and ranges of unequal length make its few nodes deeper.
-	auto four = std::async(std::launch::async, [s] {
+	auto four = std::async(n > kMaxListTris ? std::launch::async : std::launch::deferred, [s] {
 		DeviceLayout4 out;
 		if (s->tris.size() > static_cast<size_t>(kMaxListTris)) {
 			Bvh2 tree;
@@ -150,8 +150,9 @@ rn_status prepare_scene(rn_scene *s) {
 	list_triangles(s->tris, s->bvh, list);
 	RNB_CUDA(up(s->d_nodes, lay.nodes.data(), lay.nodes.size() * sizeof(F4)));
 	RNB_CUDA(up(s->d_nodes4, lay4.nodes.data(), lay4.nodes.size() * sizeof(F4)));
+	const size_t list_at = lay.tris.size(); // the list shares the triangles' buffer
+	lay.tris.insert(lay.tris.end(), list.begin(), list.end());
 	RNB_CUDA(up(s->d_tris, lay.tris.data(), lay.tris.size() * sizeof(F4)));
-	RNB_CUDA(up(s->d_list, list.data(), list.size() * sizeof(F4)));
 	RNB_CUDA(up(s->d_ref_shade, ref.data(), ref.size() * sizeof(F4)));
 	RNB_CUDA(up(s->d_phys_shade, phys.data(), phys.size() * sizeof(F4)));
 	RNB_CUDA(up(s->d_emitters, em.data(), em.size() * sizeof(F4)));
@@ -179,7 +180,7 @@ rn_status prepare_scene(rn_scene *s) {
 			edge = std::max({edge, std::fabs(static_cast<double>(t[3]) - t[0]), std::fabs(static_cast<double>(t[6]) - t[0])});
 		}
 	v.max_dir = edge > 0.0 ? static_cast<float>(std::min(3.0e38, std::ldexp(1.0, 123) / (edge * edge))) : 3.0e38f;
-	v.list = list.empty() ? nullptr : s->d_list.as<float4>();
+	v.list = list.empty() ? nullptr : s->d_tris.as<float4>() + list_at;
 	s->view = v;
 	s->prepared = true;
 	return RN_OK;

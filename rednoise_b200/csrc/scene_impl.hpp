@@ -28,7 +28,7 @@ struct rn_scene {
 
 	int device = -1;
 	cudaStream_t stream = nullptr;
-	rnb::DevBuf d_nodes, d_nodes4, d_tris, d_list, d_ref_shade, d_phys_shade, d_emitters;
+	rnb::DevBuf d_nodes, d_nodes4, d_tris, d_ref_shade, d_phys_shade, d_emitters;
 	rnb::DevBuf d_ref_geom; // ray-traced renderer: vertices and vertex normals, uploaded on first use
 	// GPU-built linear BVH (rn_pt_scene_build_lbvh), selected by RN_PT_LBVH
 	rnb::DevBuf d_lbvh_nodes, d_lbvh_tris;
