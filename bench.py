@@ -719,6 +719,9 @@ def run_ours(args):
                      "traffic": top_traffic,
                      "algorithmic": "24 B per node-box test + 36 B per triangle test of the reference-order "
                                     "closest-hit traversal, counted on the GPU for 1 spp of the same frame",
+                     "note": "the kernels walk their own tree over the reference's leaves, which rejects more with "
+                             "fewer tests than the reference's: a fraction above 1 says that these bytes are not all "
+                             "fetched; the ncu figures are of a capture over the reference's tree",
                      "kernel_ms_per_launch": top["ms_per_frame"] / args.depth,
                      "hbm": {"peak": peak, "peak_kind": peak_kind, "frac": top["frac_of_hbm"],
                              "read_probe_gbs": peaks["hbm_read_gbs"]},
