@@ -164,64 +164,12 @@ __device__ __forceinline__ unsigned dir_cell(const F3 &d) {
 	return (quantize(0.5f * (py + 1.0f), 16.0f) << 4) | quantize(0.5f * (px + 1.0f), 16.0f);
 }
 
-// Gradient sums of one block in shared memory. A few wall and emitter triangles take most
-// of the adjoint's terms, and a warp's atomics on their floats queue at the same few sectors
-// of L2; a triangle that finds its entry of this table (two places by a hash, taken by
-// whoever comes first and kept) is added up here and reaches global memory once a block, the
-// others add there at once. 512 x 512 x 32 samples of depth 6 over 1.31M triangles, whose
-// room is 12 of them: the flush of the continuation terms 7.75 -> 0.87 ms, the shadow stage
-// 5.16 -> 4.68.
-struct GradCache {
-	static constexpr int kEntries = 256;
-	static constexpr unsigned kFree = 0xffffffffu;
-	unsigned key[kEntries]; // triangle * 2 + (emission ? 1 : 0); triangles stay below 2^28
-	float sum[3 * kEntries];
-	__device__ __forceinline__ void clear() {
-		for (int i = threadIdx.x; i < kEntries; i += blockDim.x) {
-			key[i] = kFree;
-			sum[i] = sum[kEntries + i] = sum[2 * kEntries + i] = 0.0f;
-		}
-		__syncthreads();
-	}
-	__device__ __forceinline__ void add(float *base, bool emission, int tri, const F3 &v) {
-		const unsigned k = 2u * static_cast<unsigned>(tri) + (emission ? 1u : 0u);
-		const unsigned h = (k * 2654435761u) >> 24;
-#pragma unroll
-		for (unsigned p = 0; p < 2; p++) {
-			unsigned *at = key + (h ^ p);
-			unsigned have = *static_cast<volatile unsigned *>(at);
-			if (have == kFree)
-				have = atomicCAS(at, kFree, k);
-			if (have == k || have == kFree) {
-				float *q = sum + (h ^ p);
-				if (v.x != 0.0f)
-					atomicAdd(q, v.x);
-				if (v.y != 0.0f)
-					atomicAdd(q + kEntries, v.y);
-				if (v.z != 0.0f)
-					atomicAdd(q + 2 * kEntries, v.z);
-				return;
-			}
-		}
-		add_grad3(base + 3 * static_cast<size_t>(tri), v);
-	}
-	// by the whole block, after its last add
-	__device__ __forceinline__ void flush(float *d_alb, float *d_em) {
-		__syncthreads();
-		for (int i = threadIdx.x; i < kEntries; i += blockDim.x)
-			if (key[i] != kFree)
-				add_grad3(((key[i] & 1u) ? d_em : d_alb) + 3 * static_cast<size_t>(key[i] >> 1),
-				          f3(sum[i], sum[kEntries + i], sum[2 * kEntries + i]));
-	}
-};
-static_assert(GradCache::kEntries == 256, "add takes the top 8 bits of the hash");
-
 // Gradient adds of one warp merged per triangle: every lane of `mask` calls this;
-// lanes with `on` set add v to triangle tri's gradient, where add(tri, sum) puts it. Lanes
-// that share a triangle pass their values through this warp's 96 floats of shared memory
-// (scratch) to the lowest of them, which adds the sum.
-template <class Add>
-__device__ __forceinline__ void add_grad3_warp(int tri, F3 v, bool on, unsigned mask, float *scratch, Add &&add) {
+// lanes with `on` set add v to base[3 tri .. 3 tri + 2]. Lanes that share a triangle
+// pass their values through this warp's 96 floats of shared memory (scratch) to the
+// lowest of them, which adds the sum: few emitter and wall triangles take most of the
+// adjoint's terms, and one atomic per triangle and warp keeps them from queueing.
+__device__ __forceinline__ void add_grad3_warp(float *base, int tri, F3 v, bool on, unsigned mask, float *scratch) {
 	const int lane = threadIdx.x & 31;
 	const unsigned act = __ballot_sync(mask, on);
 	if (on) {
@@ -238,7 +186,7 @@ __device__ __forceinline__ void add_grad3_warp(int tri, F3 v, bool on, unsigned 
 				sum.y += scratch[32 + l];
 				sum.z += scratch[64 + l];
 			}
-			add(tri, sum);
+			add_grad3(base + 3 * static_cast<size_t>(tri), sum);
 		}
 		__syncwarp(act);
 	}
@@ -305,10 +253,8 @@ __global__ void __launch_bounds__(128, kAdj ? 5 : 7) k_wf_shade(const WfJob *__r
 		if constexpr (kAdj) {
 			__shared__ float agg[4 * 96];
 			const bool em = vg.hit_emitter >= 0;
-			// few paths hit an emitter: their sums go to global memory at once
-			add_grad3_warp(em ? vg.hit_emitter : 0, em ? g * safe_div(vg.emit, vg.Le) : f3(0.0f, 0.0f, 0.0f), em,
-			               __activemask(), agg + (threadIdx.x >> 5) * 96,
-			               [&](int tri, const F3 &v) { add_grad3(pool.d_em + 3 * static_cast<size_t>(tri), v); });
+			add_grad3_warp(pool.d_em, em ? vg.hit_emitter : 0, em ? g * safe_div(vg.emit, vg.Le) : f3(0.0f, 0.0f, 0.0f),
+			               em, __activemask(), agg + (threadIdx.x >> 5) * 96);
 		}
 		const unsigned si = warp_append(pool.counters + kCntShadow + k, sr.valid);
 		if (kBoundsCheck && sr.valid && si >= static_cast<unsigned>(pool.capacity)) {
@@ -365,12 +311,6 @@ __global__ void __launch_bounds__(128) k_wf_shadow(const WfJob *__restrict__ job
 	const unsigned n = pool.counters[kCntShadow + k];
 	const int lane = threadIdx.x & 31;
 	int err = 0;
-	GradCache *cache = nullptr;
-	if constexpr (kAdj) {
-		__shared__ GradCache block_sums;
-		cache = &block_sums;
-		cache->clear();
-	}
 	for (;;) {
 		unsigned base = 0;
 		if (lane == 0)
@@ -419,14 +359,10 @@ __global__ void __launch_bounds__(128) k_wf_shadow(const WfJob *__restrict__ job
 		if constexpr (kAdj) {
 			__shared__ float agg[4 * 96];
 			float *scratch = agg + (threadIdx.x >> 5) * 96;
-			add_grad3_warp(g_tri, g_alb_v, g_on, 0xffffffffu, scratch,
-			               [&](int tri, const F3 &v) { cache->add(pool.d_alb, false, tri, v); });
-			add_grad3_warp(g_em, g_em_v, g_on, 0xffffffffu, scratch,
-			               [&](int tri, const F3 &v) { cache->add(pool.d_em, true, tri, v); });
+			add_grad3_warp(pool.d_alb, g_tri, g_alb_v, g_on, 0xffffffffu, scratch);
+			add_grad3_warp(pool.d_em, g_em, g_em_v, g_on, 0xffffffffu, scratch);
 		}
 	}
-	if constexpr (kAdj)
-		cache->flush(pool.d_alb, pool.d_em);
 	if (err)
 		atomicOr(status, 1);
 }
@@ -785,8 +721,6 @@ cudaError_t bin_sort(const BinSrc &src, unsigned *bins, unsigned *hist, int grid
 // continuation vertex adds g (C - P) d log w / d albedo to its triangle.
 __global__ void __launch_bounds__(256) k_wf_adj_flush(const WfJob *__restrict__ jobs, WfPool pool, WfWave wave) {
 	__shared__ float agg[8 * 96];
-	__shared__ GradCache cache;
-	cache.clear();
 	float *scratch = agg + (threadIdx.x >> 5) * 96;
 	const int stride = gridDim.x * blockDim.x;
 	// the loop bound is a multiple of the block size, so whole warps run each iteration
@@ -811,11 +745,9 @@ __global__ void __launch_bounds__(256) k_wf_adj_flush(const WfJob *__restrict__ 
 				tri = __float_as_int(dl.w);
 				v = g * (C - f3(P.x, P.y, P.z)) * f3(dl.x, dl.y, dl.z);
 			}
-			add_grad3_warp(tri, v, on, 0xffffffffu, scratch,
-			               [&](int to, const F3 &sum) { cache.add(pool.d_alb, false, to, sum); });
+			add_grad3_warp(pool.d_alb, tri, v, on, 0xffffffffu, scratch);
 		}
 	}
-	cache.flush(pool.d_alb, pool.d_em);
 }
 
 // Adds each pixel's samples of this wave to its sum, in sample order.
