@@ -9,7 +9,9 @@
 #include <limits>
 #include <map>
 #include <sstream>
+#include <system_error>
 #include <thread>
+#include <utility>
 
 namespace rnb {
 
@@ -46,6 +48,27 @@ struct Shape {
 		const int v = 1 + std::max(depth_of(c / 2), depth_of(c - c / 2));
 		depth[c] = v;
 		return v;
+	}
+};
+
+// Work that may run beside its creator's: on a thread of its own, or within join() where the
+// system gives no more threads. f does not throw.
+template <class F> class Beside {
+	F f;
+	std::thread t;
+
+public:
+	explicit Beside(F g) : f(std::move(g)) {
+		try {
+			t = std::thread([this] { f(); });
+		} catch (const std::system_error &) {
+		}
+	}
+	void join() {
+		if (t.joinable())
+			t.join();
+		else
+			f();
 	}
 };
 
@@ -109,7 +132,7 @@ struct Builder {
 		node.right = r;
 		out->nodes[static_cast<size_t>(self)] = node;
 		if (par_levels > 0) {
-			std::thread left([this, l, start, nl, par_levels] { build(l, start, nl, par_levels - 1); });
+			Beside left([this, l, start, nl, par_levels] { build(l, start, nl, par_levels - 1); });
 			build(r, mid, nr, par_levels - 1);
 			left.join();
 		} else {
@@ -653,7 +676,7 @@ struct AreaTree {
 		node.left = static_cast<int>(left);
 		out.nodes[self] = node;
 		if (par_levels > 0 && j - i > 4096) {
-			std::thread first([=, this] { build(right, i, split, depth + 1, par_levels - 1); });
+			Beside first([=, this] { build(right, i, split, depth + 1, par_levels - 1); });
 			build(left, split, j, depth + 1, par_levels - 1);
 			first.join();
 		} else {

@@ -3,7 +3,11 @@
 #pragma once
 
 #include <cstdint>
+#include <future>
 #include <string>
+#include <system_error>
+#include <type_traits>
+#include <utility>
 #include <vector>
 
 namespace rnb {
@@ -142,5 +146,17 @@ void split_by_area(const Bvh2 &bvh, Bvh2 &out);
 // -(e0.x e1.z - e1.x e0.z), e0.x e1.y - e1.x e0.y, 0). Empty above kMaxListTris.
 constexpr int kMaxListTris = 128;
 void list_triangles(const TriangleSet &ts, const Bvh2 &bvh, std::vector<F4> &out);
+
+// f() on a thread of its own if `beside` is set and the system gives one, else when the future is
+// asked for its result.
+template <class F> std::future<std::invoke_result_t<F>> run_beside(bool beside, F f) {
+	if (beside) {
+		try {
+			return std::async(std::launch::async, f);
+		} catch (const std::system_error &) {
+		}
+	}
+	return std::async(std::launch::deferred, std::move(f));
+}
 
 } // namespace rnb

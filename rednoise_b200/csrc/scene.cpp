@@ -4,7 +4,6 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
-#include <future>
 #include <new>
 #include <string>
 
@@ -79,7 +78,7 @@ rn_status prepare_scene(rn_scene *s) {
 	// The 4-wide tree, while this thread lays out the reference's and the shading records. A
 	// scene of few triangles keeps the reference's shape: there is little to skip above its
 	// leaves, and ranges of unequal length make its few nodes deeper.
-	auto four = std::async(n > kMaxListTris ? std::launch::async : std::launch::deferred, [s] {
+	auto four = run_beside(n > kMaxListTris, [s] {
 		DeviceLayout4 out;
 		if (s->tris.size() > static_cast<size_t>(kMaxListTris)) {
 			Bvh2 tree;
