@@ -345,12 +345,20 @@ rn_status rn_pt_render_photon_mapped(rn_scene *scene, const rn_pt_ref_params *pr
 			p.lights[i] = to_ref_light(prm->lights[i]);
 	}
 	size_t map_bytes = 0;
-	RNB_CUDA(photon_scratch_bytes(num_photons, prm->width, prm->height, map_bytes));
+	size_t requests = photon_requests(p.width, p.height, gather_rays, false);
+	RNB_CUDA(photon_scratch_bytes(num_photons, requests, map_bytes));
 	cudaStream_t cs = pick_stream(scene, stream);
 	std::lock_guard<std::mutex> lock(scene->scratch_mu);
 	const size_t pb = (sizeof(RefParams) + 255) & ~size_t(255);
 	const size_t img = (static_cast<size_t>(npix) * 4 + 255) & ~size_t(255);
-	RNB_CUDA(scene->scratch.ensure(256 + pb + img + map_bytes));
+	cudaError_t room = scene->scratch.ensure(256 + pb + img + map_bytes);
+	if (room == cudaErrorMemoryAllocation && photon_requests(p.width, p.height, gather_rays, true) < requests) {
+		cudaGetLastError(); // the allocation's, which later calls would report again
+		requests = photon_requests(p.width, p.height, gather_rays, true);
+		RNB_CUDA(photon_scratch_bytes(num_photons, requests, map_bytes));
+		room = scene->scratch.ensure(256 + pb + img + map_bytes);
+	}
+	RNB_CUDA(room);
 	char *base = scene->scratch.as<char>();
 	int *d_err = reinterpret_cast<int *>(base);
 	RefParams *d_p = reinterpret_cast<RefParams *>(base + 256);
@@ -360,8 +368,8 @@ rn_status rn_pt_render_photon_mapped(rn_scene *scene, const rn_pt_ref_params *pr
 	RNB_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), cs));
 	RNB_CUDA(cudaMemcpyAsync(d_p, &p, sizeof(p), cudaMemcpyHostToDevice, cs));
 	unsigned stored = 0;
-	RNB_CUDA(launch_photon_mapped(scene->view, scene->d_ref_shade.as<float4>(), p, d_p, num_photons, gather_rays, d_map,
-	                              map_bytes, dev ? argb : d_argb, d_err, cs, &stored));
+	RNB_CUDA(launch_photon_mapped(scene->view, scene->d_ref_shade.as<float4>(), p, d_p, num_photons, gather_rays,
+	                              requests, d_map, map_bytes, dev ? argb : d_argb, d_err, cs, &stored));
 	if (num_stored)
 		*num_stored = stored;
 	if (!dev)

@@ -713,20 +713,21 @@ struct ReplayLeaf {
 	}
 };
 
-// Rows [y0, y1). A warp takes an 8 x 4 pixel tile, a block 16 x 8.
+// Columns [x0, x1) of rows [y0, y1). A warp takes an 8 x 4 pixel tile, a block 16 x 8.
 template <bool kList>
 __global__ void __launch_bounds__(128) k_photon_hits(SceneView sv, const float4 *__restrict__ ref_shade,
-                                                     const RefParams *__restrict__ params, PhotonRequests q, int y0,
-                                                     int y1, uint32_t *__restrict__ argb, int *status) {
+                                                     const RefParams *__restrict__ params, PhotonRequests q, int x0,
+                                                     int x1, int y0, int y1, uint32_t *__restrict__ argb,
+                                                     int *status) {
 	const RefParams &p = *params;
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	const int tiles_x = (p.width + 15) / 16;
-	const int x = static_cast<int>(blockIdx.x) % tiles_x * 16 + (warp & 1) * 8 + (lane & 7);
+	const int tiles_x = (x1 - x0 + 15) / 16;
+	const int x = x0 + static_cast<int>(blockIdx.x) % tiles_x * 16 + (warp & 1) * 8 + (lane & 7);
 	const int y = y0 + static_cast<int>(blockIdx.x) / tiles_x * 8 + (warp >> 1) * 4 + (lane >> 3);
-	if (x >= p.width || y >= y1)
+	if (x >= x1 || y >= y1)
 		return;
 	Ctx c{sv, ref_shade, &p, 0};
-	uint32_t *head = q.head + static_cast<size_t>(y - y0) * p.width + x;
+	uint32_t *head = q.head + static_cast<size_t>(y - y0) * (x1 - x0) + (x - x0);
 	const V3 dir = photon_camera_dir(p, x, y);
 	if constexpr (kList) {
 		ListLeaf leaf{q, head};
@@ -909,23 +910,26 @@ inline size_t jump_bytes(size_t max_pos, int levels, size_t n_dep) {
 
 } // namespace
 
-// Requests kept at a time: two per pixel, up to 2^24 (1.4 GB), and never fewer than one row's
-// 16 per pixel, so that a row always fits.
 constexpr uint32_t kFewRequests = 148 * 2048; // as many threads as the chip holds at once
 constexpr int kMaxHitsPerPixel = 1 << kPhotonShadeDepth;
-static size_t request_cap(int width, int height) {
-	const size_t two = 2 * static_cast<size_t>(width) * static_cast<size_t>(height);
-	return std::max(std::min(two, size_t(1) << 24), kMaxHitsPerPixel * static_cast<size_t>(width));
+size_t photon_requests(int width, int height, int gather_rays, bool fewest) {
+	if (gather_rays > 0)
+		return 0;
+	const size_t w = static_cast<size_t>(width), two = 2 * w * static_cast<size_t>(height);
+	return std::min(std::max(two, kMaxHitsPerPixel * w), size_t(1) << (fewest ? 18 : 24));
 }
-static size_t request_bytes(int width, int height, size_t &sort_bytes, cudaError_t &e) {
-	const size_t cap = request_cap(width, height);
+static size_t request_bytes(size_t cap, size_t &sort_bytes, cudaError_t &e) {
+	sort_bytes = 0;
+	e = cudaSuccess;
+	if (cap == 0)
+		return 0;
 	e = cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, static_cast<uint32_t *>(nullptr),
 	                                    static_cast<uint32_t *>(nullptr), static_cast<uint32_t *>(nullptr),
 	                                    static_cast<uint32_t *>(nullptr), static_cast<int>(cap));
 	return 4 * align256(cap * 16) + 4 * align256(cap * 4) + 256 + align256(cap * 4) + align256(sort_bytes);
 }
 
-cudaError_t photon_scratch_bytes(int n_photons, int width, int height, size_t &bytes) {
+cudaError_t photon_scratch_bytes(int n_photons, size_t requests, size_t &bytes) {
 	const size_t n_pos = static_cast<size_t>(n_photons) * kMaxDrawsPerPhoton + 8;
 	const size_t n_draws = n_pos + kMaxDrawsPerPhoton + 8;
 	int levels = 1;
@@ -947,13 +951,13 @@ cudaError_t photon_scratch_bytes(int n_photons, int width, int height, size_t &b
 	        3 * align256((static_cast<size_t>(n_photons) + 1) * 4) + 3 * align256(n_dep * 16) +
 	        2 * align256(n_dep * 8) + 2 * align256(n_dep * 4) + align256(std::max(cub_bytes, scan_bytes)) + 1024;
 	size_t sort_bytes = 0;
-	bytes += request_bytes(width, height, sort_bytes, e);
+	bytes += request_bytes(requests, sort_bytes, e);
 	return e;
 }
 
 cudaError_t launch_photon_mapped(const SceneView &sv, const float4 *ref_shade, const RefParams &hp,
-                                 const RefParams *d_params, int n_photons, int gather_rays, void *scratch,
-                                 size_t scratch_bytes, uint32_t *argb, int *status, cudaStream_t st,
+                                 const RefParams *d_params, int n_photons, int gather_rays, size_t requests,
+                                 void *scratch, size_t scratch_bytes, uint32_t *argb, int *status, cudaStream_t st,
                                  unsigned *deposits_out) {
 	const size_t max_pos = static_cast<size_t>(n_photons) * kMaxDrawsPerPhoton + 8;
 	int levels = 1;
@@ -986,17 +990,17 @@ cudaError_t launch_photon_mapped(const SceneView &sv, const float4 *ref_shade, c
 	uint32_t *d_i1 = reinterpret_cast<uint32_t *>(take(n_dep * 4));
 	size_t req_sort_bytes = 0;
 	cudaError_t e = cudaSuccess;
-	request_bytes(hp.width, hp.height, req_sort_bytes, e);
+	request_bytes(requests, req_sort_bytes, e);
 	if (e != cudaSuccess)
 		return e;
 	PhotonRequests q{};
-	const size_t cap = request_cap(hp.width, hp.height);
+	const size_t cap = requests;
 	q.cap = static_cast<uint32_t>(cap);
 	for (float4 **f : {&q.point, &q.normal, &q.albedo, &q.direct})
 		*f = reinterpret_cast<float4 *>(take(cap * 16));
 	for (uint32_t **u : {&q.key, &q.key_out, &q.order_in, &q.order, &q.head})
 		*u = reinterpret_cast<uint32_t *>(take(cap * 4));
-	q.count = reinterpret_cast<uint32_t *>(take(256));
+	q.count = reinterpret_cast<uint32_t *>(take(cap > 0 ? 256 : 0));
 	void *req_tmp = take(req_sort_bytes);
 	void *d_tmp = take(0);
 	const size_t used = static_cast<size_t>(b - static_cast<char *>(scratch));
@@ -1083,19 +1087,21 @@ cudaError_t launch_photon_mapped(const SceneView &sv, const float4 *ref_shade, c
 		                                                                         gather_rays, argb, status);
 		return cudaGetLastError();
 	}
-	// as many rows at a time as two requests a pixel allow; where more are listed, so few
-	// that no view can list more than fit
-	const int sure_rows = static_cast<int>(cap / (kMaxHitsPerPixel * static_cast<size_t>(hp.width)));
+	// strips of as many columns as a row is sure to find room for (all of them, but for rows of
+	// millions of pixels or memory that is short), and in each as many rows at a time as two
+	// requests a pixel allow; where more are listed, so few that no view can list more than fit
+	const int columns = static_cast<int>(std::min<size_t>(static_cast<size_t>(hp.width), cap / kMaxHitsPerPixel));
+	const int sure_rows = static_cast<int>(cap / (kMaxHitsPerPixel * static_cast<size_t>(columns)));
 	int rows = static_cast<int>(std::min<size_t>(static_cast<size_t>(hp.height),
-	                                             std::max<size_t>(cap / (2 * static_cast<size_t>(hp.width)),
+	                                             std::max<size_t>(cap / (2 * static_cast<size_t>(columns)),
 	                                                              static_cast<size_t>(sure_rows))));
-	for (int y0 = 0; y0 < hp.height;) {
-		const int y1 = std::min(hp.height, y0 + rows);
-		const unsigned blocks = static_cast<unsigned>((hp.width + 15) / 16) * static_cast<unsigned>((y1 - y0 + 7) / 8);
+	for (int x0 = 0, y0 = 0; x0 < hp.width;) {
+		const int x1 = std::min(hp.width, x0 + columns), y1 = std::min(hp.height, y0 + rows);
+		const unsigned blocks = static_cast<unsigned>((x1 - x0 + 15) / 16) * static_cast<unsigned>((y1 - y0 + 7) / 8);
 		e = cudaMemsetAsync(q.count, 0, 4, st);
 		if (e != cudaSuccess)
 			return e;
-		k_photon_hits<true><<<blocks, 128, 0, st>>>(sv, ref_shade, d_params, q, y0, y1, argb, status);
+		k_photon_hits<true><<<blocks, 128, 0, st>>>(sv, ref_shade, d_params, q, x0, x1, y0, y1, argb, status);
 		uint32_t n = 0;
 		e = cudaMemcpyAsync(&n, q.count, 4, cudaMemcpyDeviceToHost, st);
 		if (e != cudaSuccess)
@@ -1120,8 +1126,10 @@ cudaError_t launch_photon_mapped(const SceneView &sv, const float4 *ref_shade, c
 			const unsigned whole = std::min<unsigned>(n, kBlockGathers), lanes = n - whole;
 			k_photon_gather<<<whole + static_cast<unsigned>(ceil_div(static_cast<long>(lanes), bs)), bs, 0, st>>>(m, q, n);
 		}
-		k_photon_hits<false><<<blocks, 128, 0, st>>>(sv, ref_shade, d_params, q, y0, y1, argb, status);
-		y0 = y1;
+		k_photon_hits<false><<<blocks, 128, 0, st>>>(sv, ref_shade, d_params, q, x0, x1, y0, y1, argb, status);
+		y0 = y1 < hp.height ? y1 : 0;
+		if (y0 == 0)
+			x0 = x1;
 	}
 	return cudaGetLastError();
 }
