@@ -112,12 +112,30 @@ __device__ __forceinline__ V3 hemisphere_direction(const Frame &f, V3 local) {
 	return normalize(f.t * local.x + f.b * local.y + f.n * local.z);
 }
 
+// intersect() by trace_closest4_flat.
+__device__ __forceinline__ Hit intersect_flat(Ctx &c, V3 o, V3 d) {
+	const RayPre r = make_ray(o.x, o.y, o.z, d.x, d.y, d.z);
+	HitRec h;
+	if (c.sv.nodes4 && bounded_ray(c.sv, r)) {
+		LocalStack<unsigned long long> st;
+		h = trace_closest4_flat(c.sv, r, -1, c.err, st);
+	} else {
+		h = trace_closest<kOrderReference>(c.sv, r, -1, c.err);
+	}
+	Hit out;
+	out.hit = h.idx >= 0;
+	out.idx = h.idx;
+	out.t = h.t;
+	out.point = o + h.t * d;
+	return out;
+}
+
 // tracePath (src/BDPT.cpp:43-61): the path's vertices, position and 2 * triangle + 1 if
 // faceViewer flipped the normal (the throughputs follow from the triangles, see replay).
-template <class D> __device__ int gi_subpath(Ctx &c, V3 o, V3 d, float4 *out, D &draw) {
+template <bool kFlat, class D> __device__ int gi_subpath(Ctx &c, V3 o, V3 d, float4 *out, D &draw) {
 	int k = 0;
 	for (; k < kGiMaxDepth; k++) {
-		const Hit h = intersect(c, o, d, -1);
+		const Hit h = kFlat ? intersect_flat(c, o, d) : intersect(c, o, d, -1);
 		if (!h.hit)
 			break;
 		const V3 tn = tri_normal(c.ref_shade, h.idx);
@@ -149,14 +167,14 @@ template <class D> __device__ V3 emitter_point(D &draw) {
 // Both subpaths as kBdptRecordSlots vertices: the camera's from slot 0 on, the point on the
 // emitter in slot 4 and the light's vertices after it. Returns the two lengths (hits), the
 // camera's in the low four bits.
-template <class D>
+template <bool kFlat, class D>
 __device__ int bdpt_subpaths(Ctx &c, const GiParams &p, const GiCam &cam, int x, int y, D &draw, float4 *v) {
 	const V3 dir = camera_direction(p, cam, x, y, draw);
-	const int nc = gi_subpath(c, cam.pos, dir, v, draw);
+	const int nc = gi_subpath<kFlat>(c, cam.pos, dir, v, draw);
 	const V3 lp = emitter_point(draw);
 	v[kGiMaxDepth] = make_float4(lp.x, lp.y, lp.z, 0.0f);
 	const V3 ldir = hemisphere_direction(hemisphere_frame(mk(0.0f, -1.0f, 0.0f)), draw.local());
-	return nc | (gi_subpath(c, lp + kGiEps * ldir, ldir, v + kGiMaxDepth + 1, draw) << 4);
+	return nc | (gi_subpath<kFlat>(c, lp + kGiEps * ldir, ldir, v + kGiMaxDepth + 1, draw) << 4);
 }
 constexpr int kBdptMinDraws = 6;                                  // a sample that hits nothing
 constexpr int kBdptMaxDraws = kBdptMinDraws + 4 * kGiMaxDepth;    // both subpaths of full length
@@ -458,7 +476,7 @@ __global__ void __launch_bounds__(kT *kStride, 1) k_bdpt_rows(SceneView sv, cons
 		int lengths = 0;
 		if (start && px < x1) {
 			RingDraw<kT * kStride> draw{rs, read + 2 * t};
-			lengths = bdpt_subpaths(c, p, cam, px, y, draw, v);
+			lengths = bdpt_subpaths<true>(c, p, cam, px, y, draw, v);
 		}
 		if (start) {
 			next[t] = kBdptMinDraws + 2 * ((lengths & 15) + (lengths >> 4));
@@ -511,7 +529,7 @@ __global__ void __launch_bounds__(128) k_bdpt_counter_paths(SceneView sv, const 
 	CtrDraw d{static_cast<uint32_t>(pix), static_cast<uint32_t>(s), 0u, static_cast<uint32_t>(p.seed),
 	          static_cast<uint32_t>(p.seed >> 32), 0, U4{0u, 0u, 0u, 0u}};
 	float4 v[kBdptRecordSlots];
-	const int lengths = bdpt_subpaths(c, p, gi_cam(p), x, y, d, v);
+	const int lengths = bdpt_subpaths<false>(c, p, gi_cam(p), x, y, d, v);
 	write_record(v, lengths, rec, cnt, static_cast<size_t>(i));
 	if (c.err)
 		atomicOr(status, 1);
@@ -964,10 +982,18 @@ int bdpt_chunk_width(const GiParams &p, size_t budget) {
 // warps, 39.7 with three, 43.6 with four; 153 rows: 1.96, 1.88, 1.80). Sixteen or eight
 // lanes a ray were slower at every number of paths (45.8 ms and more): a ray's chain gets
 // longer by more than the fewer warps give back.
-// k_bdpt_rows: with one or two samples a pixel, the assumed pixels are wrong sooner, so
-// half the starts are traced, each on four times the lanes' room (an 82 000-triangle
-// sphere, 278 x 271 x 2: <64, 4> 31.2 ms, <128, 1> 36.4, one thread a row 39.5; 1 300
-// triangles, 500 x 450 x 4: 91.9, 58.4 and 91.3 ms).
+// k_bdpt_rows: with few samples a pixel the assumed pixels are wrong sooner, so half the starts
+// are traced, each with twice the room. Milliseconds of <64, 2> and <128, 1>, and of a thread a row
+// over the tree before:
+//   width x rows x samples      96x64x3          120x480x2         120x480x4
+//   128 random + 1 triangles    3.92 4.15  9.1   6.30 5.94 10.2    10.5 9.22 20.4
+//   20 000 random triangles     31.9 29.9 44.1   47.2 42.7 48.0    86.1 73.1 95.3
+//   1 300-triangle sphere       4.82 5.33 11.9   7.98 8.05 13.9    13.3 13.1 27.0
+//   82 000-triangle sphere      6.96 8.00 17.5   11.1 11.2 20.9    18.7 18.9 41.8
+// (one sample a pixel, 96 x 64: 2.27 2.63 3.20, 14.5 16.4 15.2, 2.61 3.94 4.12, 3.94 6.05 6.07;
+// 120 x 480, 20 000 random triangles: 25.8 25.2 24.2, the one case found where a thread a row
+// was faster). Other numbers of starts and lanes, 1 to 128 by 1 to 32, were slower but for <32, 8>
+// at 64 rows of one sample (2.07, 12.7, 2.46, 3.23).
 void launch_rows(const SceneView &sv, const float4 *ref_shade, const GiParams &p, const RowStreams &rs, int x0, int x1,
                  float4 *rec, uint8_t *cnt, int *status, cudaStream_t st) {
 	const unsigned rows = static_cast<unsigned>(p.height);
@@ -975,8 +1001,8 @@ void launch_rows(const SceneView &sv, const float4 *ref_shade, const GiParams &p
 		k_bdpt_rows_list<32, 4><<<rows, 128, 0, st>>>(sv, ref_shade, p, rs, x0, x1, rec, cnt, status);
 	else if (sv.list)
 		k_bdpt_rows_list<32, 2><<<rows, 64, 0, st>>>(sv, ref_shade, p, rs, x0, x1, rec, cnt, status);
-	else if (p.samples <= 2)
-		k_bdpt_rows<64, 4><<<rows, 256, 0, st>>>(sv, ref_shade, p, rs, x0, x1, rec, cnt, status);
+	else if (p.samples <= 3)
+		k_bdpt_rows<64, 2><<<rows, 128, 0, st>>>(sv, ref_shade, p, rs, x0, x1, rec, cnt, status);
 	else
 		k_bdpt_rows<128, 1><<<rows, 128, 0, st>>>(sv, ref_shade, p, rs, x0, x1, rec, cnt, status);
 }

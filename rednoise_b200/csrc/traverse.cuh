@@ -671,6 +671,81 @@ __device__ __forceinline__ HitRec trace_closest4_spec(const SceneView &s, const 
 	return h;
 }
 
+// Closest hit in the reference's order for lanes with little company (the row streams of the
+// bidirectional renderer, where one candidate start in eight is taken): nothing is postponed, and a
+// leaf's triangles, up to four at a time, are loaded together and tested as independent
+// straight-line work, then merged in leaf order. 120 x 480 x 4 samples over 20 000 random
+// triangles: 99.5 -> 73 ms, over a 20 000-triangle sphere 18.4 -> 16.8.
+template <class Stack>
+__device__ __forceinline__ HitRec trace_closest4_flat(const SceneView &s, const RayPre &r, int ignore, int &err,
+                                                      Stack &st) {
+	const RayPair r2 = make_pair_ray(r);
+	HitRec h;
+	h.idx = -1;
+	h.rank = 0x7fffffff;
+	h.t = __int_as_float(0x7f800000);
+	h.u = 0.0f;
+	h.v = 0.0f;
+	int sp = 0;
+	float te;
+	if (s.n_tris > 0 && slab(s.root_lo[0], s.root_hi[0], s.root_lo[1], s.root_hi[1], s.root_lo[2], s.root_hi[2], r, te)) {
+		st.put(0, pack_entry(s.root4_ref, te));
+		sp = 1;
+	}
+	while (sp > 0) {
+		const unsigned long long e = st.get(--sp);
+		int ref = static_cast<int>(static_cast<unsigned>(e));
+		if (!(__int_as_float(static_cast<int>(e >> 32)) < h.t))
+			continue;
+		while (ref >= 0) {
+			if (bad_node(s, ref, true) || sp + 3 > kStack) {
+				err = 1;
+				return h;
+			}
+			float t[4];
+			bool b[4];
+			int4 rf;
+			node4_test(s, ref, r2, t, b, rf);
+			if (b[3])
+				st.put(sp++, pack_entry(rf.w, t[3]));
+			if (b[2])
+				st.put(sp++, pack_entry(rf.z, t[2]));
+			if (b[1])
+				st.put(sp++, pack_entry(rf.y, t[1]));
+			ref = b[0] && t[0] < h.t ? rf.x : kNoRef;
+		}
+		if (ref == kNoRef)
+			continue;
+		const int start = leaf_start(ref), count = leaf_count(ref);
+		if (bad_leaf(s, start, count)) {
+			err = 1;
+			return h;
+		}
+		for (int at = 0; at < count; at += 4) {
+			float4 ta[4], tb[4], tc[4];
+#pragma unroll
+			for (int q = 0; q < 4; q++) {
+				const float4 *tp = s.tris + 3 * static_cast<size_t>(start + min(at + q, count - 1));
+				ta[q] = __ldg(tp + 0);
+				tb[q] = __ldg(tp + 1);
+				tc[q] = __ldg(tp + 2);
+			}
+#pragma unroll
+			for (int q = 0; q < 4; q++) {
+				float t, u, v;
+				const bool ok = tri_test<true, true>(ta[q], tb[q], tc[q], r, t, u, v) & (at + q < count) &
+				                (__float_as_int(ta[q].w) != ignore) & (t < h.t);
+				h.idx = ok ? __float_as_int(ta[q].w) : h.idx;
+				h.t = ok ? t : h.t;
+				h.u = ok ? u : h.u;
+				h.v = ok ? v : h.v;
+				h.rank = ok ? __float_as_int(tc[q].w) : h.rank;
+			}
+		}
+	}
+	return h;
+}
+
 // ---- one ray by a group of lanes, for scenes of few triangles ----
 // A lone ray's traversal is a chain of dependent loads and tests: 5 000 to 20 000 cycles in
 // a scene of 36 triangles. Where rays are few, or come one after another, a group of
