@@ -124,12 +124,21 @@ __global__ void __launch_bounds__(128) k_trace_any_group(SceneView s, int n, con
 
 // kGroup lanes per ray up to this many rays, a thread per ray beyond: closest and any hits of
 // the 36-triangle box take 6 us of device time for 4 096 rays (39 with a thread per ray), 12
-// (40) for 16 384, 31 (45) for 65 536 and 62 (56) for 131 072.
+// (40) for 16 384, 31 (45) for 65 536 and 62 (56) for 131 072. At the list's end, 128
+// triangles, 65 536 rays take 41 and 37 us where a thread per ray over 129 takes 43 and 34.
 constexpr int kGroupRays = 1 << 16;
-// Closest hits of this many rays and more, over larger scenes, take the persistent kernel: below
-// it too few warps have a ray to go on with (65 536 rays over 1.31M triangles 180 us, 201
-// with it; 262 144 over 82 000 triangles 216 and 207; 2M over 1.31M 1 081 and 884; now 778).
-constexpr int kStreamRays = 1 << 17;
+// Closest hits of this many rays and more, over scenes of this many triangles and more, take the
+// persistent kernel. Below, too few warps have a ray to go on with, or the rays are too alike in
+// length to repay the exchange. Time with a thread per ray over time with it:
+//   rays                       131 072  262 144  2M
+//   128 random + 1 triangles   0.95     0.90     0.83
+//   512                        0.92     1.00     0.97
+//   1 000                      0.92     1.00     1.01
+//   5 000                      0.95     1.11     1.20
+//   1 300-triangle sphere      0.85     1.03     1.10
+//   20 500                     0.98     1.07     1.26
+//   1.31M                      0.99     1.02     1.38 (1.12 -> 0.82 ms)
+constexpr int kStreamRays = 1 << 18, kStreamTris = 768;
 
 cudaError_t launch_trace_closest(const SceneView &v, int n, const float *o, const float *d, const int *ignore,
                                  int order, int *tri, float *t, float *u, float *vv, int *err, cudaStream_t st) {
@@ -141,7 +150,7 @@ cudaError_t launch_trace_closest(const SceneView &v, int n, const float *o, cons
 		                                                                                  vv, err);
 	else if (order == kOrderNearest)
 		k_trace_closest<kOrderNearest><<<ceil_div(n, bs), bs, 0, st>>>(v, n, o, d, ignore, tri, t, u, vv, err);
-	else if (v.nodes4 && !v.list && n >= kStreamRays)
+	else if (v.nodes4 && v.n_tris >= kStreamTris && n >= kStreamRays)
 		k_trace_closest_stream<<<148 * kStreamBlocks, bs, kStreamSmem, st>>>(v, n, o, d, ignore, tri, t, u, vv, err);
 	else
 		k_trace_closest<kOrderReference><<<ceil_div(n, bs), bs, 0, st>>>(v, n, o, d, ignore, tri, t, u, vv, err);
