@@ -162,10 +162,12 @@ void build_reference_bvh(const float *v9, int n, Bvh2 &out) {
 	if (n > 0) {
 		out.nodes.resize(static_cast<size_t>(b.shape.node_count(n)));
 		out.depth = b.shape.depth_of(n);
-		// Threads only where subtrees are large enough to repay them.
+		// Threads only where subtrees are large enough to repay them: of 2048 triangles on (16
+		// cores; 5 000 random triangles 1.03 -> 0.43 ms, 15 000 3.4 -> 1.1, 50 000 13.2 -> 3.4
+		// against those of 65 536 on; 4096 0.61, 1.3 and 2.9).
 		const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
 		int par = 0;
-		while ((1u << par) < 2 * hw && (n >> par) > 65536)
+		while ((1u << par) < 2 * hw && (n >> par) > 2048)
 			par++;
 		b.build(0, 0, n, par);
 		out.root = 0;
