@@ -733,8 +733,8 @@ __device__ __forceinline__ HitRec trace_closest4_flat(const SceneView &s, const 
 #pragma unroll
 			for (int q = 0; q < 4; q++) {
 				float t, u, v;
-				const bool ok = tri_test<true, true>(ta[q], tb[q], tc[q], r, t, u, v) & (at + q < count) &
-				                (__float_as_int(ta[q].w) != ignore) & (t < h.t);
+				const bool hit = tri_test<true, true>(ta[q], tb[q], tc[q], r, t, u, v);
+				const bool ok = hit & (at + q < count) & (__float_as_int(ta[q].w) != ignore) & (t < h.t);
 				h.idx = ok ? __float_as_int(ta[q].w) : h.idx;
 				h.t = ok ? t : h.t;
 				h.u = ok ? u : h.u;
@@ -868,7 +868,8 @@ __device__ __forceinline__ bool trace_any_group(const SceneView &s, const TriLis
 	} else {
 		for (int j = g; j < s.n_tris; j += kGroup) {
 			float te, t, u, v;
-			any |= list.test(j, r, ignore, te, t, u, v) & (te < tmax) & (t < tmax);
+			const bool hit = list.test(j, r, ignore, te, t, u, v);
+			any |= hit & (te < tmax) & (t < tmax);
 		}
 	}
 	return (__ballot_sync(0xffffffffu, any) & (group_lanes<kGroup>() << (lane - g))) != 0;
