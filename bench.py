@@ -165,6 +165,15 @@ class ClockSampler:
 
 # ---- CPU baseline: the reference's renderPathTraced (oracle/_ref) ---------------------
 
+NO_REFERENCE = {"unavailable": "oracle/_ref/librn_ref.so is not built here (it needs the reference's sources)"}
+
+
+def reference_available() -> bool:
+    import oracle
+
+    return oracle.ref_available()
+
+
 def reference_model(sc):
     import oracle
 
@@ -218,6 +227,8 @@ def reference_rate(model, w, h, spp, calls, warmup=0, min_s=0.0, full_spp=64) ->
 
 
 def cpu_baseline(sc, w=1920, h=1080, target_s=12.0) -> dict:
+    if not reference_available():
+        return {"unit": UNIT, "cores": os.cpu_count(), "kind": "reference", **NO_REFERENCE}
     model = reference_model(sc)
     r = reference_rate(model, w, h, 2, calls=1, min_s=target_s)
     return {"value": r["value"], "unit": UNIT, "cores": os.cpu_count(), "kind": "reference",
@@ -380,6 +391,9 @@ def time_to_rmse(scene, lib, stream, sptr, cam, args, fp64, W, H, target=0.5, fr
 def run_reference_arm(args):
     rank, _, world = dist_env()
     if rank != 0:
+        return
+    if not reference_available():
+        print(json.dumps({"impl": "reference", **NO_REFERENCE}), flush=True)
         return
     from rednoise_b200 import scenes
 
@@ -758,9 +772,10 @@ def run_ours(args):
         line["cpu_baseline"] = cpu_baseline(sc)
         line["cpu_physical_fp32"] = cpu_physical_baseline(sc, c, args)
         line["like_for_like"] = {
-            "reference_semantics": {"gpu_samples_per_s": like_for_like["value"],
-                                    "reference_cpu_samples_per_s": line["cpu_baseline"]["value"],
-                                    "speedup": like_for_like["value"] / line["cpu_baseline"]["value"]},
+            "reference_semantics": NO_REFERENCE if "unavailable" in line["cpu_baseline"] else
+            {"gpu_samples_per_s": like_for_like["value"],
+             "reference_cpu_samples_per_s": line["cpu_baseline"]["value"],
+             "speedup": like_for_like["value"] / line["cpu_baseline"]["value"]},
             "physical_estimator": {"gpu_samples_per_s": value,
                                    "oracle_fp32_cpu_samples_per_s": line["cpu_physical_fp32"]["value"],
                                    "speedup": value / line["cpu_physical_fp32"]["value"]}}
@@ -977,21 +992,23 @@ def run_raytraced(args):
     for _ in range(args.steps):
         s.render_raytraced(W, H, focal_length=focal, position=pos)
     gpu_s = (time.perf_counter() - t0) / args.steps
-    model = reference_model(sc)
-    w, h = W, H
-    t0 = time.perf_counter()
-    model.render_raytraced(w, h, focal=reference_focal(h), pos=pos)
-    cpu_s = time.perf_counter() - t0
-    build = reference_bvh_build_s(model)
-    cpu_rate = w * h / max(cpu_s - build, 1e-9)
+    cpu = NO_REFERENCE
+    if reference_available():
+        model = reference_model(sc)
+        t0 = time.perf_counter()
+        model.render_raytraced(W, H, focal=focal, pos=pos)
+        cpu_s = time.perf_counter() - t0
+        build = reference_bvh_build_s(model)
+        cpu = {"value": W * H / max(cpu_s - build, 1e-9), "unit": "pixels/s", "cores": os.cpu_count(),
+               "kind": "reference",
+               "sample": f"reference renderRaytraced, one {W}x{H} frame of the same camera ({cpu_s:.1f} s, its BVH "
+                         f"rebuild of {build:.2f} s excluded)"}
     line = {"metric": "pixels/s (Whitted ray tracing, end to end through the C ABI)", "value": W * H / gpu_s,
             "unit": "pixels/s", "n_gpus": 1, "steps": args.steps, "warmup": args.warmup, "ms_per_step": gpu_s * 1e3,
             "higher_is_better": True, "dtype": "f32", "data": "synthetic",
             "config": {"workload": f"icosphere-cornell-1.31M-tris {W}x{H} renderRaytraced (Phong, default light, "
                                    "depth 4)", "output": "host canvas, copy included"},
-            "cpu_baseline": {"value": cpu_rate, "unit": "pixels/s", "cores": os.cpu_count(), "kind": "reference",
-                             "sample": f"reference renderRaytraced, one {w}x{h} frame of the same camera "
-                                       f"({cpu_s:.1f} s, its BVH rebuild of {build:.2f} s excluded)"}}
+            "cpu_baseline": cpu}
     print(json.dumps(line), flush=True)
 
 
@@ -1020,22 +1037,25 @@ def run_photon(args):
     for _ in range(args.steps):
         img, stored = s.render_photon_mapped(W, H, photons, focal_length=focal, position=pos, return_count=True)
     gpu_s = (time.perf_counter() - t0) / args.steps
-    model = reference_model(sc)
-    t0 = time.perf_counter()
-    want = model.render_photon_mapped(W, H, photons, focal=focal, pos=pos)
-    cpu_s = time.perf_counter() - t0
-    build = reference_bvh_build_s(model)
-    same = float((img == want).mean())
+    same, cpu = None, NO_REFERENCE
+    if reference_available():
+        model = reference_model(sc)
+        t0 = time.perf_counter()
+        want = model.render_photon_mapped(W, H, photons, focal=focal, pos=pos)
+        cpu_s = time.perf_counter() - t0
+        build = reference_bvh_build_s(model)
+        same = float((img == want).mean())
+        cpu = {"value": 1.0 / max(cpu_s - build, 1e-9), "unit": "frames/s", "cores": os.cpu_count(),
+               "kind": "reference",
+               "sample": f"reference renderPhotonMapped, one frame ({cpu_s:.1f} s, its BVH rebuild of {build:.2f} s "
+                         f"excluded)"}
     line = {"metric": "frames/s (photon mapping, end to end through the C ABI)", "value": 1.0 / gpu_s,
             "unit": "frames/s", "n_gpus": 1, "steps": args.steps, "warmup": args.warmup, "ms_per_step": gpu_s * 1e3,
             "higher_is_better": True, "dtype": "f32", "data": "synthetic",
             "config": {"workload": f"icosphere-cornell-1.31M-tris {W}x{H} renderPhotonMapped, {photons} photons",
                        "stored_photons": stored, "output": "host canvas, copy included"},
             "identical_pixels_vs_reference": same,
-            "cpu_baseline": {"value": 1.0 / max(cpu_s - build, 1e-9), "unit": "frames/s", "cores": os.cpu_count(),
-                             "kind": "reference",
-                             "sample": f"reference renderPhotonMapped, one frame ({cpu_s:.1f} s, its BVH rebuild of "
-                                       f"{build:.2f} s excluded)"}}
+            "cpu_baseline": cpu}
     print(json.dumps(line), flush=True)
 
 
@@ -1086,9 +1106,22 @@ def cornell_pair():
     s = rn.Scene.from_arrays(a["cornell_v"], ref_rgb=a["cornell_rgb"], ref_material=a["cornell_material"],
                              ref_normal=a["cornell_normal"], ref_roughness=a["cornell_roughness"])
     s.prepare()
-    m = oracle.RefModel.from_arrays(a["cornell_v"], a["cornell_rgb"], a["cornell_material"], a["cornell_roughness"],
-                                    a["cornell_normal"])
+    m = None
+    if reference_available():
+        m = oracle.RefModel.from_arrays(a["cornell_v"], a["cornell_rgb"], a["cornell_material"],
+                                        a["cornell_roughness"], a["cornell_normal"])
     return s, m
+
+
+def reference_frame(m, render, what):
+    """(canvas, CPU figures) of one frame by the reference; no canvas where it is not built."""
+    if m is None:
+        return None, NO_REFERENCE
+    t0 = time.perf_counter()
+    want = render(m)
+    cpu_s = time.perf_counter() - t0
+    return want, {"value": 1.0 / cpu_s, "unit": "frames/s", "cores": os.cpu_count(), "kind": "reference",
+                  "sample": f"{what}, one frame ({cpu_s:.2f} s)"}
 
 
 def time_calls(fn, warmup, steps):
@@ -1112,20 +1145,18 @@ def run_bidirectional(args):
     W, H, spp = (160, 120, 16) if args.small else (640, 480, 64)
     ref_s, img = time_calls(lambda: s.render_bidirectional(W, H, spp), args.warmup, args.steps)
     ctr_s, _ = time_calls(lambda: s.render_bidirectional(W, H, spp, rng="counter"), args.warmup, args.steps)
-    t0 = time.perf_counter()
-    want = m.render_bidirectional(W, H, spp)
-    cpu_s = time.perf_counter() - t0
+    want, cpu = reference_frame(m, lambda m: m.render_bidirectional(W, H, spp),
+                                "reference renderBidirectional (oracle/_ref, OpenMP)")
     line = {"metric": "frames/s (bidirectional path tracing, end to end through the C ABI)", "value": 1.0 / ref_s,
             "unit": "frames/s", "n_gpus": 1, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ref_s * 1e3,
             "higher_is_better": True, "dtype": "f32", "data": "reference asset (Cornell box, 32 triangles)",
             "config": {"workload": f"cornell-box {W}x{H} renderBidirectional, {spp} spp, exposure 40, camera (0,0,4)",
                        "rng": "reference per-row std::mt19937 streams", "output": "host canvas, copy included"},
             "samples_per_s": W * H * spp / ref_s,
-            "identical_pixels_vs_reference": float((img == want).mean()),
+            "identical_pixels_vs_reference": None if want is None else float((img == want).mean()),
             "counter_stream": {"value": 1.0 / ctr_s, "unit": "frames/s", "ms_per_step": ctr_s * 1e3,
                                "samples_per_s": W * H * spp / ctr_s},
-            "cpu_baseline": {"value": 1.0 / cpu_s, "unit": "frames/s", "cores": os.cpu_count(), "kind": "reference",
-                             "sample": f"reference renderBidirectional (oracle/_ref, OpenMP), one frame ({cpu_s:.2f} s)"}}
+            "cpu_baseline": cpu}
     print(json.dumps(line), flush=True)
 
 
@@ -1141,9 +1172,8 @@ def run_metropolis(args):
     W, H, muts = (160, 120, 400000) if args.small else (640, 480, 4000000)
     gpu_s, img = time_calls(lambda: s.render_metropolis(W, H, muts), args.warmup, args.steps)
     big_s, _ = time_calls(lambda: s.render_metropolis(W, H, 16 * muts), 1, 1)
-    t0 = time.perf_counter()
-    want = m.render_metropolis(W, H, muts)
-    cpu_s = time.perf_counter() - t0
+    want, cpu = reference_frame(m, lambda m: m.render_metropolis(W, H, muts),
+                                "reference renderMetropolis (oracle/_ref, 16 OpenMP chains)")
     ch = lambda c: np.stack([(c >> 16) & 255, (c >> 8) & 255, c & 255], -1).astype(np.float64)  # noqa: E731
     line = {"metric": "frames/s (Metropolis light transport, end to end through the C ABI)", "value": 1.0 / gpu_s,
             "unit": "frames/s", "n_gpus": 1, "steps": args.steps, "warmup": args.warmup, "ms_per_step": gpu_s * 1e3,
@@ -1153,11 +1183,9 @@ def run_metropolis(args):
                        "chains": muts // 16, "output": "host canvas, copy included"},
             "mutations_per_s": muts / gpu_s,
             "mutations_per_s_64M": 16 * muts / big_s,
-            "mean_level": {"gpu": float(ch(img).mean()), "reference": float(ch(want).mean())},
-            "mean_abs_level_difference_vs_reference": float(np.abs(ch(img) - ch(want)).mean()),
-            "cpu_baseline": {"value": 1.0 / cpu_s, "unit": "frames/s", "cores": os.cpu_count(), "kind": "reference",
-                             "sample": f"reference renderMetropolis (oracle/_ref, 16 OpenMP chains), one frame "
-                                       f"({cpu_s:.2f} s)"}}
+            "mean_level": {"gpu": float(ch(img).mean()), "reference": None if want is None else float(ch(want).mean())},
+            "mean_abs_level_difference_vs_reference": None if want is None else float(np.abs(ch(img) - ch(want)).mean()),
+            "cpu_baseline": cpu}
     print(json.dumps(line), flush=True)
 
 
