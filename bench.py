@@ -690,25 +690,27 @@ def run_ours(args):
 
     peak, peak_kind = measured_peaks()
     kernel_ms = float(np.mean(render_ms))
-    achieved = bytes_per_sample * samples_per_step / (kernel_ms / 1e3) / 1e9
     kp = kernel_profile() or {}
-    # DRAM bytes of the frame's three stage kernels (about 93 % of its device time),
+    # DRAM bytes of the frame's three stage kernels (88 % of its device time),
     # per sample from the committed ncu capture of the same scene at 480x270
     stage_bps = sum(kp[k]["dram_bytes_per_sample"] for k in ("k_wf_extend", "k_wf_shadow", "k_wf_shade") if k in kp)
     traffic = stage_bps * samples_per_step if stage_bps else None
-    # Traversal kernels against the level that holds their working set (the 4-wide tree
-    # and the triangles, ~150 MB, mostly L1/L2-resident): algorithmic bytes of the
-    # reference traversal per stage over the stage's device time.
-    ext_bps = (24.0 * counts["closest_boxes"] + 36.0 * counts["closest_tris"]) / counts["samples"]
-    sh_bps = (24.0 * counts["any_boxes"] + 36.0 * counts["any_tris"]) / counts["samples"]
+    # Traversal kernels against the level that holds most of their working set (the 4-wide
+    # tree and the triangles, ~150 MB): the bytes they read from L2, per sample from the
+    # same capture. Beside them the work that the reference's traversal would do for these
+    # rays (24 B per node-box test, 36 B per triangle test), which is not what is fetched.
+    ext_ref = (24.0 * counts["closest_boxes"] + 36.0 * counts["closest_tris"]) / counts["samples"]
+    sh_ref = (24.0 * counts["any_boxes"] + 36.0 * counts["any_tris"]) / counts["samples"]
     per_kernel = {}
-    for name, bps, ms_key in (("k_wf_extend", ext_bps, "extend_ms"), ("k_wf_shadow", sh_bps, "shadow_ms")):
+    for name, ref_bps, ms_key in (("k_wf_extend", ext_ref, "extend_ms"), ("k_wf_shadow", sh_ref, "shadow_ms")):
         ms = stages[ms_key]
-        gbs = bps * samples_per_step / (ms / 1e3) / 1e9 if ms > 0 else None
+        l2_bps, dram_bps = (kp.get(name, {}).get(k) for k in ("l2_read_bytes_per_sample", "dram_bytes_per_sample"))
+        rate = lambda bps: bps * samples_per_step / (ms / 1e3) / 1e9 if bps and ms > 0 else None  # noqa: E731
         ent = {"ms_per_frame": ms, "launches_per_frame": args.depth, "share_of_frame": ms / stages["total_ms"],
-               "algorithmic_bytes_per_sample": bps, "achieved_gbs": gbs,
-               "frac_of_l2_read": gbs / peaks["l2_read_gbs"] if gbs else None,
-               "frac_of_hbm": gbs / peak if gbs else None}
+               "l2_read_bytes_per_sample": l2_bps, "achieved_gbs": rate(l2_bps),
+               "frac_of_l2_read": rate(l2_bps) / peaks["l2_read_gbs"] if rate(l2_bps) else None,
+               "frac_of_hbm": rate(dram_bps) / peak if rate(dram_bps) else None,
+               "reference_traversal_bytes_per_sample": ref_bps}
         if name in kp:
             ent["ncu"] = {k: v for k, v in kp[name].items() if k != "per_launch"}
         per_kernel[name] = ent
@@ -727,20 +729,17 @@ def run_ours(args):
         "gpu_launches": launches_per_step * args.steps,
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": ctypes.sizeof(cam) + ctypes.sizeof(st),
                 "d2h_bytes_per_step": H * W * 3 * 4, "api": "rn_pt_render with host output buffer"},
-        "roofline": {"bound": "l2", "kernel": "k_wf_extend", "achieved": top["achieved_gbs"],
+        "roofline": {"bound": "issue", "kernel": "k_wf_extend", "achieved": top["achieved_gbs"],
                      "peak": peaks["l2_read_gbs"], "unit": "GB/s", "frac": top["frac_of_l2_read"],
                      "peak_kind": "measured in this run: L2-resident read (rn_pt_probe_read, loads bypassing L1)",
                      "traffic": top_traffic,
-                     "algorithmic": "24 B per node-box test + 36 B per triangle test of the reference-order "
-                                    "closest-hit traversal, counted on the GPU for 1 spp of the same frame",
-                     "note": "the kernels walk their own tree over the reference's leaves, which rejects more with "
-                             "fewer tests than the reference's: a fraction above 1 says that these bytes are not all "
-                             "fetched; the ncu figures are of a capture over the reference's tree",
+                     "bytes": "read from L2 by the closest-hit stage, per sample from the committed ncu capture of the "
+                              "same scene at 480x270, over the stage's device time in this run; the stage is bound by "
+                              "instruction issue and divergence (see issue), not by L2 or HBM",
                      "kernel_ms_per_launch": top["ms_per_frame"] / args.depth,
                      "hbm": {"peak": peak, "peak_kind": peak_kind, "frac": top["frac_of_hbm"],
                              "read_probe_gbs": peaks["hbm_read_gbs"]},
-                     "issue": ({"bound_by": "L1 throughput and instruction issue (profiles/traversal_kernels_*.md, "
-                                            "profiles/k_wf_extend_*.md)",
+                     "issue": ({"bound_by": "instruction issue and divergence (profiles/traversal_kernels_*.md)",
                                 "issue_active_pct": kp["k_wf_extend"]["issue_active_pct"],
                                 "issue_active_pct_bounces_0_2": float(np.mean(
                                     [l["issue_pct"] for l in kp["k_wf_extend"]["per_launch"][:3]])),
@@ -748,9 +747,9 @@ def run_ours(args):
                                if "k_wf_extend" in kp else None),
                      "per_kernel": per_kernel,
                      "stages_ms": stages,
-                     "frame": {"achieved": achieved, "bytes_per_sample": bytes_per_sample, "kernel_ms": kernel_ms,
-                               "frac_of_l2_read": achieved / peaks["l2_read_gbs"], "frac_of_hbm": achieved / peak,
-                               "dram_traffic_stage_kernels": traffic},
+                     "frame": {"kernel_ms": kernel_ms, "dram_traffic_stage_kernels": traffic,
+                               "frac_of_hbm": traffic / (kernel_ms / 1e3) / 1e9 / peak if traffic else None,
+                               "reference_traversal_bytes_per_sample": bytes_per_sample},
                      "probes": peaks},
         "time_to_rmse": t_rmse,
         "clocks": clk,
