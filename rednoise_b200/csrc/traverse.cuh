@@ -155,7 +155,7 @@ __device__ __forceinline__ bool slab(float lox, float hix, float loy, float hiy,
 // edges side by side and their products are formed in pairs. (Expressions are the
 // reference's with signs moved, which changes no bit: -(x * y) and (-x) * y are the same, and so
 // are (-x) - (-y) and y - x.)
-// A ray takes 10 to 14 of these tests, with 18 to 20 of a warp's lanes in step, and a warp
+// A ray takes 11 to 14 of these tests, with 16 to 18 of a warp's lanes in step, and a warp
 // rarely leaves at an early exit of its lanes: between the determinant and t there is one,
 // behind u and v together, and the 4-wide traversals load the whole record before they look
 // at the index to ignore. Against the reference's order of tests and unpaired products: the
